@@ -201,7 +201,8 @@ __global__ __launch_bounds__(1024) void bin_colscan_kernel(uint32_t* __restrict_
             uint32_t base = 0;
             if (tx == leader) base = atomicAdd(words + 8u + k, __popc(m));
             base = __shfl_sync(0xffffffffu, base, leader);
-            if (cls == k) lists[k * tiles + base + __popc(m & lanemask_lt())] = t;
+            // Lanes past the last tile are of the empty class too: not filed.
+            if (valid && cls == k) lists[k * tiles + base + __popc(m & lanemask_lt())] = t;
         }
     }
     __syncthreads();
