@@ -149,10 +149,12 @@ int sf_scratch_reserve(sf_scratch s, uint64_t isects);
 /* Kernel forms a scratch launches; all forms give identical results (the
  * autotuner picks by measured time). */
 typedef struct {
-    uint32_t raster_cull; /* 0: every warp walks every staged entry;
-                             1: per-warp culling by each splat's power_max box,
-                             then by the minimum of its quadratic form over
-                             the warp's 8x4 pixel block */
+    /* Which walk the pair diagnostics (raster_detail) count: 0, every warp
+     * walks every staged entry; 1, per-warp culling by each splat's power_max
+     * box, then by the minimum of its quadratic form over the warp's 8x4
+     * pixel block. Without raster_detail every frame culls, whichever value
+     * is set. */
+    uint32_t raster_cull;
     /* Intersection build, same lists either way:
      *   SF_ISECTS_BINNED (default, frames up to 49152 tiles): per-tile
      *     counts in shared memory, place, then a sort of each tile's list by
@@ -212,9 +214,8 @@ int sf_scratch_set_tuning(sf_scratch s, const sf_tuning* t);
 int sf_scratch_get_tuning(sf_scratch s, sf_tuning* t);
 /* Frame autotuner (no counterpart in the reference): times sf_render_frames
  * over cams[count] at w x h for each raster form in a coordinate search (two
- * sweeps over raster_cull {0,1}, raster_split {1,2,4}, raster_order {sorted,
- * hybrid, in-raster}, raster_schedule {longest, tiles} and frame_pipes
- * {2, 1}; best of three
+ * sweeps over raster_split {1,2,4}, raster_order {sorted, hybrid, in-raster},
+ * raster_schedule {longest, tiles} and frame_pipes {2, 1}; best of three
  * paths after a warm-up path), keeps the fastest on the scratch and returns
  * it with its time per frame. Images are the same in every form. */
 int sf_scratch_autotune(sf_splats s, sf_scratch scratch, const sf_camera* cams, uint32_t count, uint32_t w,
@@ -285,9 +286,9 @@ int sf_render_backward(sf_splats s, sf_scratch scratch, const sf_camera* cam, ui
  * mask(p) into fg[i] and with dL/dF(p) = 1 - mask(p) into bg[i] (device
  * [n] floats; mask NULL: all of it in fg) — the real-valued mask and
  * background responsibilities sum_p m_p alpha_i T_i(p), which the u32 lift
- * truncates per pixel to (u32)(alpha T scale). A transmittance-only forward
- * keeps each pixel's final T and last contributor; the adjoint replays the
- * sorted lists back to front from them. Float sums, added in no fixed order.
+ * truncates per pixel to (u32)(alpha T scale). Both factors are at hand in the
+ * forward walk, so one pass over the sorted lists sums them (and keeps each
+ * pixel's final T and last contributor). Float sums, added in no fixed order.
  * Syncs once (the intersection total). Overwrites an sf_render_forward's
  * state on the scratch. */
 int sf_render_feature_adjoint(sf_splats s, sf_scratch scratch, const sf_camera* cam, uint32_t w, uint32_t h,
@@ -415,7 +416,7 @@ int sf_table_entropy(sf_ctx ctx, const float* a, const float* b, uint32_t n, flo
 typedef struct sf_round_t* sf_round;
 typedef struct {
     uint32_t lanes;       /* capture streams the views are spread over (1..64) */
-    uint32_t raster_cull; /* as sf_tuning.raster_cull */
+    uint32_t raster_cull; /* kept, without effect: every round culls per warp */
     uint32_t isect_build; /* as sf_tuning.isect_build */
     uint32_t raster_order; /* as sf_tuning.raster_order */
     uint32_t raster_split; /* as sf_tuning.raster_split */
@@ -451,11 +452,11 @@ int sf_round_evidence(sf_round r, sf_splats s, sf_beta beta, const sf_camera* ca
 int sf_round_evidence_words(sf_round r, uint32_t view, const uint32_t** fg, const uint32_t** bg);
 /* Adjoint evidence round (no counterpart in the reference): every view's
  * responsibilities from the adjoint of a per-splat scalar feature
- * (sf_render_feature_adjoint: transmittance-only forward, back-to-front
- * replay) in the round's graph, real-valued fg / bg per splat (masks NULL,
- * or a NULL entry: all of the view in fg), and with beta each view's EIG
- * over fg + bg (sf_beta_eig_real). Syncs once. The lists are sorted for the
- * replay whatever the tuning's raster_order. */
+ * (sf_render_feature_adjoint) in the round's graph, real-valued fg / bg per
+ * splat (masks NULL, or a NULL entry: all of the view in fg), and with beta
+ * each view's EIG
+ * over fg + bg (sf_beta_eig_real). Syncs once. The lists are sorted
+ * whatever the tuning's raster_order. */
 int sf_round_evidence_adjoint(sf_round r, sf_splats s, sf_beta beta, const sf_camera* cams,
                               const sf_mask* masks, int mode, sf_stream stream, double* eig);
 /* View `view` of the last adjoint round: device fg and bg floats [total]. */
@@ -463,8 +464,7 @@ int sf_round_adjoint_responsibility(sf_round r, uint32_t view, const float** fg,
 /* Autotuner (the round's kernel forms picked by measured time): a
  * coordinate search, two sweeps, over lanes {1,2,4,8}, isect_build {binned,
  * depth-sorted}, raster_order {sorted, in-raster, hybrid} (binned build),
- * raster_cull {0,1}, raster_split {1,2,4} (rasterizer warps per CTA 8, 4
- * or 2 on 16x16 tiles) and radix_bits {4,6,8} (sort digit width, depth-sorted
+ * raster_split {1,2,4} (rasterizer warps per CTA 8, 4 or 2 on 16x16 tiles) and radix_bits {4,6,8} (sort digit width, depth-sorted
  * build), each candidate timed as the best of three rounds
  * after a warm-up round. The winner and its time stay on the round and in
  * a process-wide cache keyed by (device, splats, view sizes, kind); a cached

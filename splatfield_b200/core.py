@@ -565,7 +565,8 @@ class RenderScratch:
     def set_tuning(self, raster_cull: int = 0, isect_build: int = L.ISECTS_BINNED, raster_detail: int = 0,
                    raster_order: int = L.ORDER_SORTED, raster_schedule: int = L.SCHEDULE_LONGEST,
                    raster_split: int = 1, radix_bits: int = 8, frame_pipes: int = 2) -> None:
-        """Kernel forms (results are identical across forms): raster_cull 0/1,
+        """Kernel forms (results are identical across forms): raster_cull 0/1
+        (which walk raster_detail counts; frames always cull per warp),
         isect_build ISECTS_BINNED (default) or ISECTS_DEPTH_SORTED,
         raster_detail 1 to count the per-pair diagnostics of ``stats``,
         raster_order ORDER_SORTED (default), ORDER_IN_RASTER or ORDER_HYBRID,

@@ -625,7 +625,6 @@ int frame_graph_capture(sf_splats sp, sf_scratch s) {
         a.geo1 = s->geo1;
         a.color = s->color;
         a.ext = s->ext;
-        a.cull = s->tuning.raster_cull;
         a.split = s->tuning.raster_split;
         a.stats = s->stats;
         a.bitmap = s->bitmap;
@@ -1347,7 +1346,7 @@ int sf_render_feature_adjoint(sf_splats s, sf_scratch scratch, const sf_camera* 
         if (!s || !scratch || !cam || !fg || !bg) return fail(SF_ERR_ARG, "null argument");
         if (mask && (mask->w != w || mask->h != h)) return fail(SF_ERR_SHAPE, "mask size does not match the frame");
         cudaStream_t st = S(stream);
-        // Sorted lists: the adjoint replays them back to front.
+        // Sorted lists: the scratch is left with a whole prepared frame.
         int rc = prepare(s, scratch, cam, w, h, st, nullptr);
         if (rc != SF_OK) return rc;
         const size_t pixels = (size_t)w * h;
@@ -1357,26 +1356,14 @@ int sf_render_feature_adjoint(sf_splats s, sf_scratch scratch, const sf_camera* 
         RasterArgs a = raster_args(scratch, nullptr);
         a.final_t = scratch->final_t;
         a.n_contrib = scratch->n_contrib;
+        a.mask = mask ? mask->bits : nullptr;
+        a.mask_wpr = mask ? mask->wpr : 0u;
+        a.afg = fg;
+        a.abg = bg;
         SF_CK(cudaMemsetAsync(scratch->stats, 0, 32, st));
-        SF_CK(launch_raster(3, a, st));
         SF_CK(cudaMemsetAsync(fg, 0, (size_t)s->n * 4, st));
         SF_CK(cudaMemsetAsync(bg, 0, (size_t)s->n * 4, st));
-        FeatureBwdArgs f{};
-        f.w = w;
-        f.h = h;
-        f.tiles_x = scratch->tiles_x;
-        f.tiles_y = scratch->tiles_y;
-        f.tile_start = scratch->tile_start;
-        f.gaussian_ids = scratch->gids;
-        f.geo0 = scratch->geo0;
-        f.geo1 = scratch->geo1;
-        f.final_t = scratch->final_t;
-        f.n_contrib = scratch->n_contrib;
-        f.mask = mask ? mask->bits : nullptr;
-        f.mask_wpr = mask ? mask->wpr : 0u;
-        f.fg = fg;
-        f.bg = bg;
-        SF_CK(launch_feature_bwd(f, st));
+        SF_CK(launch_raster(3, a, st));
         return SF_OK;
     })
 }
@@ -1471,16 +1458,15 @@ static int scratch_autotune(sf_splats s, sf_scratch scratch, const sf_camera* ca
         float winner_ms = 1e30f;
         int rc = time_of(winner, &winner_ms);
         if (rc != SF_OK) return rc;
-        const uint32_t vals[5][3] = {{0, 1, 0}, {1, 2, 4}, {SF_ORDER_SORTED, SF_ORDER_HYBRID, SF_ORDER_IN_RASTER},
+        const uint32_t vals[4][3] = {{1, 2, 4}, {SF_ORDER_SORTED, SF_ORDER_HYBRID, SF_ORDER_IN_RASTER},
                                      {SF_SCHEDULE_LONGEST, SF_SCHEDULE_TILES, 0}, {2, 1, 0}};
-        const int nvals[5] = {2, 3, 3, 2, 2};
+        const int nvals[4] = {3, 3, 2, 2};
         for (int sweep = 0; sweep < 2; ++sweep)
-            for (int dim = 0; dim < 5; ++dim)
+            for (int dim = 0; dim < 4; ++dim)
                 for (int k = 0; k < nvals[dim]; ++k) {
                     sf_tuning t = winner;
-                    uint32_t* field = dim == 0 ? &t.raster_cull : dim == 1 ? &t.raster_split
-                                    : dim == 2 ? &t.raster_order : dim == 3 ? &t.raster_schedule
-                                                                            : &t.frame_pipes;
+                    uint32_t* field = dim == 0 ? &t.raster_split : dim == 1 ? &t.raster_order
+                                    : dim == 2 ? &t.raster_schedule : &t.frame_pipes;
                     if (*field == vals[dim][k]) continue;
                     *field = vals[dim][k];
                     float ms = 0.f;

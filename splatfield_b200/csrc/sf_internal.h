@@ -107,10 +107,12 @@ struct RasterArgs {
     uint32_t* resp;
     uint32_t* fg;
     uint32_t* bg;
+    float* afg;  // mode 3: real-valued responsibilities, added to
+    float* abg;
     float* final_t;
     uint32_t* n_contrib;
-    // Raster form: 0 walks every staged entry in every warp, 1 culls per warp
-    // block with the power_max boxes (needs ext).
+    // Form of the detail walk: 0 visits every staged entry in every warp, 1
+    // culls per warp block. Without detail every walk culls.
     uint32_t cull;
     // CTAs per 16x16 tile (0 or 1: one CTA of 8 warps; 2 or 4: CTAs of 4 or
     // 2 warps, each walking the whole list for its part of the pixels).
@@ -127,8 +129,9 @@ struct RasterArgs {
     const uint32_t* class_lists;
     const uint32_t* class_n;
 };
-// mode 0 = RGB, 1 = total responsibility, 2 = evidence, 3 = transmittance
-// only (final_t and n_contrib required).
+// mode 0 = RGB, 1 = total responsibility, 2 = evidence, 3 = real-valued fg /
+// bg responsibilities (afg[i] += sum_p mask(p) alpha_i T_i(p), abg[i] += sum_p
+// (1 - mask(p)) alpha_i T_i(p); mask null: all in afg). ext is always needed.
 cudaError_t launch_raster(int mode, const RasterArgs& a, cudaStream_t stream);
 
 // Adjoint (sf_backward.cu).
@@ -145,24 +148,6 @@ struct BwdArgs {
     float* d2d;                // [n][9] accumulated: mean2d xy, conic xyz, rgb, opacity
 };
 cudaError_t launch_raster_bwd(const BwdArgs& a, cudaStream_t stream);
-// Adjoint of a per-splat scalar feature: fg[i] += sum_p mask(p) alpha_i
-// T_i(p), bg[i] += sum_p (1 - mask(p)) alpha_i T_i(p) (mask null: all in
-// fg), replayed from the state of the transmittance-only raster (mode 3)
-// over the same sorted lists.
-struct FeatureBwdArgs {
-    uint32_t w, h, tiles_x, tiles_y;
-    const uint32_t* tile_start;
-    const uint32_t* gaussian_ids;
-    const float4* geo0;
-    const float4* geo1;
-    const float* final_t;
-    const uint32_t* n_contrib;
-    const uint32_t* mask;
-    uint32_t mask_wpr;
-    float* fg;
-    float* bg;
-};
-cudaError_t launch_feature_bwd(const FeatureBwdArgs& a, cudaStream_t stream);
 cudaError_t launch_project_bwd(const sf_view& view, const float* attr, const float* sh, uint32_t n,
                                uint32_t sh_per_ch, const float* d2d, float* d_attr, float* d_sh,
                                cudaStream_t stream);

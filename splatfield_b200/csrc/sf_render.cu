@@ -192,18 +192,26 @@ __device__ __forceinline__ bool project_one(const sf_view& v, const float* __res
     o.geo0[i] = make_float4(mx, my, 0.5f * cx, cy);
     o.geo1[i] = make_float4(0.5f * cz, opacity, power_max, 0.0f);
     if (o.ext) {
-        // Half extents of the box around {power <= P}, P = power_max with a
-        // 1e-4 margin for rounding: for q = hx dx^2 + hz dy^2 + cy dx dy the
-        // level set's x extent is sqrt(P * hz / det), det = hx hz - cy^2/4.
+        // Half extents of the box around {power <= P}: for q = hx dx^2 +
+        // hz dy^2 + cy dx dy the level set's x extent is sqrt(P * hz / det),
+        // det = hx hz - cy^2/4 (each product's rounding error kept, since the
+        // difference cancels in a long thin form). P is power_max with a
+        // margin for the rounding of the rasterizer's power, which is a few
+        // 2^-24 of the sum of |terms|: at the box's edge that sum is at most
+        // 4 P hx hz / det, and further out it grows no faster than the power.
         // Outside the box the computed power exceeds power_max, so the
         // rasterizer may skip the pair. A degenerate form gets no box.
         const float hx = 0.5f * cx, hz = 0.5f * cz;
-        const float dq = hx * hz - 0.25f * (cy * cy);
-        const float P = power_max * 1.0001f + 1e-4f;
+        const float hc = 0.5f * cy, cc2 = hc * hc;
+        const float dq = fma_(hx, hz, -cc2) - fma_(hc, hc, -cc2);
+        const float slack = 1.0f - 4e-6f * (hx * hz / dq);
         float ex = INFINITY, ey = INFINITY;
-        if (dq > 0.0f && P > 0.0f) {
-            ex = sqrtf(P * hz / dq) * 1.0001f + 1e-3f;
-            ey = sqrtf(P * hx / dq) * 1.0001f + 1e-3f;
+        if (dq > 0.0f && slack > 0.5f) {
+            const float P = (power_max * 1.0001f + 1e-4f) / slack;
+            if (P > 0.0f) {
+                ex = sqrtf(P * hz / dq) * 1.0001f + 1e-3f;
+                ey = sqrtf(P * hx / dq) * 1.0001f + 1e-3f;
+            }
         }
         o.ext[i] = make_float2(ex, ey);
     }

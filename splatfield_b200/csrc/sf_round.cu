@@ -77,9 +77,6 @@ struct RoundLane {
     uint32_t *tid_e = nullptr, *gid_e = nullptr, *tid_a = nullptr, *gid_a = nullptr;  // gid_a: tid_a + cap
     uint32_t* tile_start = nullptr;
     double* partials = nullptr;
-    // Adjoint round: the transmittance-only forward's per-pixel state.
-    float* final_t = nullptr;
-    uint32_t* n_contrib = nullptr;
     // Binned build: [chunks][max_tiles] histogram, per-tile totals, class lists.
     uint32_t* hist = nullptr;
     uint32_t* cnt = nullptr;
@@ -118,7 +115,6 @@ struct sf_round_t {
     bool adjoint = false;
     float* afg = nullptr;
     float* abg = nullptr;
-    uint64_t max_pixels = 0;
     uint32_t eig_blocks = 1;
     uint64_t want_cap = 0;
     // graph cache
@@ -130,7 +126,7 @@ struct sf_round_t {
     const void* g_beta = nullptr;
     int g_mode = -1;
     int g_adjoint = -1;
-    uint32_t g_lanes = 0, g_cull = 0, g_build = 0, g_order = 0, g_split = 0, g_radix = 0;
+    uint32_t g_lanes = 0, g_build = 0, g_order = 0, g_split = 0, g_radix = 0;
     // Per view: the longest tile list of the last round, and whether the
     // graph includes the segmented sort of the longest lists for the view.
     std::vector<uint32_t> longest;
@@ -149,7 +145,7 @@ void lane_free(RoundLane& L) {
     L.scan_tmp = L.sort_tmp = nullptr;
     dfree(L.tid_e); dfree(L.gid_e); dfree(L.tid_a);
     L.gid_a = nullptr;
-    dfree(L.tile_start); dfree(L.partials); dfree(L.final_t); dfree(L.n_contrib);
+    dfree(L.tile_start); dfree(L.partials);
     dfree(L.hist); dfree(L.cnt); dfree(L.lists);
     dfree(L.giant.ctrl); dfree(L.giant.sel); dfree(L.giant.mm); dfree(L.giant.hist);
     dfree(L.giant.taken); dfree(L.giant.segs);
@@ -172,8 +168,6 @@ cudaError_t lane_alloc(sf_round_t* r, RoundLane& L, uint64_t cap) {
     L.gid_a = L.tid_a + cap;
     RA(L.tile_start, (size_t)r->max_tiles + 1);
     RA(L.partials, r->eig_blocks);
-    RA(L.final_t, r->max_pixels);
-    RA(L.n_contrib, r->max_pixels);
     if (r->max_tiles <= kBinMaxTiles) {
         RA(L.hist, (size_t)r->chunks * r->max_tiles);
         RA(L.cnt, (size_t)r->max_tiles + 1);
@@ -274,7 +268,6 @@ cudaError_t raster_and_eig(sf_round_t* r, RoundLane& L, uint32_t v, uint32_t tx,
     a.geo0 = L.geo0;
     a.geo1 = L.geo1;
     a.ext = L.ext;
-    a.cull = r->tuning.raster_cull;
     a.split = r->tuning.raster_split;
     a.scale = (float)((uint64_t)1 << frac_bits(w, h));
     if (bg) {
@@ -297,9 +290,8 @@ cudaError_t raster_and_eig(sf_round_t* r, RoundLane& L, uint32_t v, uint32_t tx,
     return cudaSuccess;
 }
 
-// Adjoint round, view v: the transmittance-only raster keeps each pixel's
-// final T and last contributor, the feature adjoint replays them into the
-// view's real-valued fg / bg responsibilities, and the EIG reads fg + bg.
+// Adjoint round, view v: the raster's real-valued fg / bg responsibilities
+// and, with a posterior, the EIG over fg + bg.
 cudaError_t adjoint_and_eig(sf_round_t* r, RoundLane& L, uint32_t v, uint32_t tx, uint32_t ty,
                             const uint32_t* gids, const float* beta_a, const float* beta_b, const float* lut,
                             int mode, cudaStream_t st) {
@@ -319,28 +311,14 @@ cudaError_t adjoint_and_eig(sf_round_t* r, RoundLane& L, uint32_t v, uint32_t tx
     a.geo0 = L.geo0;
     a.geo1 = L.geo1;
     a.ext = L.ext;
-    a.cull = r->tuning.raster_cull;
-    a.final_t = L.final_t;
-    a.n_contrib = L.n_contrib;
-    if ((e = launch_raster(3, a, st)) != cudaSuccess) return e;
+    a.split = r->tuning.raster_split;
+    a.mask = mask ? mask->bits : nullptr;
+    a.mask_wpr = mask ? mask->wpr : 0u;
+    a.afg = fg;
+    a.abg = bg;
     if ((e = cudaMemsetAsync(fg, 0, (size_t)n * 4, st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(bg, 0, (size_t)n * 4, st)) != cudaSuccess) return e;
-    FeatureBwdArgs f{};
-    f.w = w;
-    f.h = h;
-    f.tiles_x = tx;
-    f.tiles_y = ty;
-    f.tile_start = L.tile_start;
-    f.gaussian_ids = gids;
-    f.geo0 = L.geo0;
-    f.geo1 = L.geo1;
-    f.final_t = L.final_t;
-    f.n_contrib = L.n_contrib;
-    f.mask = mask ? mask->bits : nullptr;
-    f.mask_wpr = mask ? mask->wpr : 0u;
-    f.fg = fg;
-    f.bg = bg;
-    if ((e = launch_feature_bwd(f, st)) != cudaSuccess) return e;
+    if ((e = launch_raster(3, a, st)) != cudaSuccess) return e;
     if (beta_a)
         return launch_eig_real(mode, beta_a, beta_b, fg, bg, n, lut, L.partials, r->eig_blocks, r->eig_dev + v, st,
                                r->h0);
@@ -359,7 +337,7 @@ cudaError_t enqueue_view(sf_round_t* r, RoundLane& L, uint32_t v, const sf_splat
     const uint32_t tiles = tx * ty;
     cudaError_t e;
     if ((e = cudaMemsetAsync(words, 0, 64, st)) != cudaSuccess) return e;
-    ProjOut po{L.keys, L.counts, L.bbox, L.geo0, L.geo1, nullptr, words, r->tuning.raster_cull ? L.ext : nullptr};
+    ProjOut po{L.keys, L.counts, L.bbox, L.geo0, L.geo1, nullptr, words, L.ext};
     sf_view dummy{};
     if ((e = launch_project(dummy, sp.attr, sp.geom, sp.sh, n, sp.K, po, st, r->views_dev + v)) != cudaSuccess) return e;
     const uint32_t *tids = nullptr, *gids = nullptr;
@@ -378,7 +356,7 @@ cudaError_t enqueue_view(sf_round_t* r, RoundLane& L, uint32_t v, const sf_splat
                                   pairs, words + 1, st)) != cudaSuccess)
             return e;
         if ((e = launch_clamp_starts(L.tile_start, tiles + 1, (uint32_t)L.cap, st)) != cudaSuccess) return e;
-        // The adjoint replays sorted lists: every class is sorted for it.
+        // The adjoint's lists are sorted whatever the tuning's order.
         const uint32_t order = r->adjoint ? SF_ORDER_SORTED : r->tuning.raster_order;
         if (order != SF_ORDER_SORTED) lazy_pairs = pairs;
         if (order != SF_ORDER_IN_RASTER) {
@@ -466,7 +444,6 @@ int build_graph(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, int
     r->g_mode = mode;
     r->g_adjoint = (int)r->adjoint;
     r->g_lanes = (uint32_t)r->lanes.size();
-    r->g_cull = r->tuning.raster_cull;
     r->g_build = r->tuning.isect_build;
     r->g_order = r->tuning.raster_order;
     r->g_split = r->tuning.raster_split;
@@ -494,7 +471,7 @@ int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const
         }
         if (!r->exec || r->g_splats != sp || r->g_beta != beta || r->g_mode != mode ||
             r->g_adjoint != (int)r->adjoint ||
-            r->g_cull != r->tuning.raster_cull || r->g_build != r->tuning.isect_build ||
+            r->g_build != r->tuning.isect_build ||
             r->g_order != r->tuning.raster_order || r->g_split != r->tuning.raster_split ||
             r->g_radix != r->tuning.radix_bits || r->g_masks != r->masks ||
             giant_changed(r)) {
@@ -571,7 +548,6 @@ int sf_round_create(sf_ctx ctx, uint32_t total, uint32_t n_views, const uint32_t
     r->g_giant.assign(n_views, 0u);
     for (uint32_t v = 0; v < n_views; ++v) {
         r->max_tiles = std::max(r->max_tiles, ((widths[v] + 15) / 16) * ((heights[v] + 15) / 16));
-        r->max_pixels = std::max<uint64_t>(r->max_pixels, (uint64_t)widths[v] * heights[v]);
     }
     r->eig_blocks = eig_blocks(total, ctx->sm_count);
     r->chunks = bin_chunks(total, ctx->sm_count);
@@ -795,25 +771,24 @@ int autotune(sf_round r, sf_splats s, sf_beta beta, const sf_camera* cams, const
     if (rc != SF_OK) return rc;
     if (winner.radix_bits == 0) winner.radix_bits = 8;
     const std::vector<uint32_t> lanes_v = {1, 2, 4, 8}, build_v = {SF_ISECTS_BINNED, SF_ISECTS_DEPTH_SORTED},
-                                order_v = {SF_ORDER_SORTED, SF_ORDER_IN_RASTER, SF_ORDER_HYBRID}, cull_v = {0, 1},
+                                order_v = {SF_ORDER_SORTED, SF_ORDER_IN_RASTER, SF_ORDER_HYBRID},
                                 split_v = {1, 2, 4}, radix_v = {4, 6, 8};
     for (int sweep = 0; sweep < 2; ++sweep) {
-        for (int dim = 0; dim < 6; ++dim) {
+        for (int dim = 0; dim < 5; ++dim) {
             const std::vector<uint32_t>& vals = dim == 0 ? lanes_v : dim == 1 ? build_v : dim == 2 ? order_v
-                                              : dim == 3 ? cull_v : dim == 4 ? split_v : radix_v;
+                                              : dim == 3 ? split_v : radix_v;
             for (uint32_t val : vals) {
                 sf_round_tuning t = winner;
                 uint32_t* field = dim == 0 ? &t.lanes : dim == 1 ? &t.isect_build : dim == 2 ? &t.raster_order
-                                : dim == 3 ? &t.raster_cull : dim == 4 ? &t.raster_split : &t.radix_bits;
+                                : dim == 3 ? &t.raster_split : &t.radix_bits;
                 if (*field == val) continue;
                 *field = val;
                 if (dim == 0 && val > r->views) continue;
-                // The orders apply to the binned build; the adjoint replays
-                // sorted lists, and its transmittance pass runs one CTA per tile.
+                // The orders apply to the binned build; the adjoint walks
+                // sorted lists.
                 if (dim == 2 && (t.isect_build != SF_ISECTS_BINNED || kind == SF_ROUND_ADJOINT)) continue;
-                if (dim == 4 && kind == SF_ROUND_ADJOINT) continue;
                 // The digit width applies to the depth-sorted build's sorts.
-                if (dim == 5 && t.isect_build != SF_ISECTS_DEPTH_SORTED) continue;
+                if (dim == 4 && t.isect_build != SF_ISECTS_DEPTH_SORTED) continue;
                 if (dim == 1 && val == SF_ISECTS_DEPTH_SORTED) t.raster_order = SF_ORDER_SORTED;
                 float ms = 0.f;
                 rc = time_of(t, &ms);
