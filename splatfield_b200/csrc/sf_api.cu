@@ -1328,6 +1328,7 @@ int sf_render_backward(sf_splats s, sf_scratch scratch, const sf_camera* cam, ui
         a.geo0 = scratch->geo0;
         a.geo1 = scratch->geo1;
         a.color = scratch->color;
+        a.ext = scratch->ext;
         a.final_t = scratch->final_t;
         a.n_contrib = scratch->n_contrib;
         a.dl = reinterpret_cast<const float4*>(dl_drgba);

@@ -142,6 +142,7 @@ struct BwdArgs {
     const float4* geo0;
     const float4* geo1;
     const float4* color;
+    const float2* ext;
     const float* final_t;      // forward's final transmittance per pixel
     const uint32_t* n_contrib; // forward's 1-based last contributor per pixel
     const float4* dl;          // dL/d(r, g, b, a) per pixel
