@@ -7,11 +7,13 @@
 //  * one upfront kernel reads the keys once and builds the 256-bin histogram
 //    of every 8-bit digit position;
 //  * one kernel per digit: a partition of 4096 keys (8192 from 2M keys on)
-//    is ranked in registers and shared memory (stable warp ranking by one
-//    ballot per digit bit), publishes its digit
-//    counts, resolves its global digit offsets by decoupled look-back over the
-//    preceding partitions, and scatters through shared memory so each digit's
-//    run is written contiguously.
+//    is ranked in registers and shared memory (stable warp ranking by lane
+//    masks), publishes its digit counts, goes into shared memory in sorted
+//    order, resolves its global digit offsets by decoupled look-back over the
+//    preceding partitions, and is written out, each digit's run contiguously.
+//    10M random pairs, 32 bits: 0.440 -> 0.313 ms for the whole sort (1M 89 ->
+//    75 us, 1k 50 -> 44 us) against ballot ranking with the look-back before
+//    the shared scatter and one shared counter per histogram bin.
 // Partition indices come from an atomic ticket in launch order, so a block
 // only ever waits on blocks that already hold a ticket (forward progress).
 // Every wait is bounded: after kSpinLimit polls the block records
@@ -37,14 +39,12 @@ constexpr int kWarps = kThreads / 32;
 // Digit passes: partitions of THREADS x 16 keys. The look-back chain across
 // partitions bounds a large pass (a partition publishes its inclusive prefix
 // only after its own look-back), so from kWidePassN keys on the partitions
-// are 8192 keys of 512 threads (half the chain: 10M keys 0.47 -> 0.44 ms);
+// are 8192 keys of 512 threads (half the chain);
 // smaller sorts keep 4096-key partitions of 256 threads, whose single
 // partitions finish sooner (1k-500k keys 12-17% faster than the wide form).
 // The keys and values staged for the scatter are dynamic shared memory.
 constexpr uint32_t kWidePassN = 1u << 21;
 constexpr int kMinPassTile = 256 * kItems;  // look-back space is sized for it
-template <int THREADS>
-constexpr size_t pass_smem() { return 2 * (size_t)THREADS * kItems * 4; }
 constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagPrefix = 2u << 30;
 constexpr uint32_t kCountMask = (1u << 30) - 1u;
@@ -77,54 +77,73 @@ __device__ __forceinline__ void st_relaxed64(unsigned long long* p, unsigned lon
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-__device__ __forceinline__ uint32_t ld_status(const uint32_t* p) { return ld_relaxed(p); }
-__device__ __forceinline__ unsigned long long ld_status(const unsigned long long* p) {
-    return ld_relaxed64(p);
-}
-
-// Decoupled look-back from partition `part` over status words stat[p * stride]
-// (flag in the top two bits: 0 = not ready, aggregate, inclusive prefix).
-// kWindow predecessors are loaded at once, so a chain of aggregates costs one
-// L2 round trip per kWindow partitions instead of one per partition. Returns
-// the exclusive prefix. A poll that finds nothing new backs off with
-// __nanosleep (32 ns, doubling to 256 ns), so waiting blocks leave issue
-// slots and L2 bandwidth to the partitions still ranking (10M-key sorts
-// 0.52 -> 0.49 ms); a wait that outlasts kSpinLimit polls (about a second
-// with the naps) records SF_DEV_ERR_TIMEOUT and returns what it has.
-constexpr int kWindow = 8;
-template <typename W>
-__device__ __forceinline__ W lookback_window(const W* stat, size_t stride, uint32_t part, W flag_prefix,
-                                             W value_mask, uint32_t* err, uint32_t spin_limit) {
-    W excl = 0;
-    int64_t p = (int64_t)part - 1;
-    uint32_t spins = 0, nap = 32;
+// Decoupled look-back from partition `part` over one digit's status words
+// stat[p * stride] (flag in the top two bits: 0 = not ready, aggregate,
+// inclusive prefix), by the LPD lanes of a warp that share the digit: slot s
+// (this lane's place among them) reads the kWindow predecessors after the
+// kWindow * s nearest ones, so one L2 round trip covers LPD * kWindow
+// partitions. All partitions of a wave publish their aggregates at about the
+// same time, so a partition i places into the wave waits about
+// i / (2 LPD kWindow) round trips for its prefix, and this chain is what
+// bounds a large pass. Every lane of the group returns the exclusive prefix.
+// A poll that finds nothing new backs off with __nanosleep (32 ns, doubling
+// to 256 ns), so waiting blocks leave issue slots and L2 bandwidth to the
+// partitions still ranking; a wait that outlasts kSpinLimit polls (about a
+// second with the naps) records SF_DEV_ERR_TIMEOUT and returns what it has.
+// Every lane of the warp must call it (the groups leave the loop together).
+constexpr int kWindow = 4;
+template <int LPD>
+__device__ __forceinline__ uint32_t lookback_digit(const uint32_t* stat, size_t stride, uint32_t part, bool active,
+                                                   uint32_t* err, uint32_t spin_limit) {
+    static_assert(LPD == 1 || LPD == 2, "lanes per digit");
+    const uint32_t slot = LPD == 2 ? (threadIdx.x & 31u) >> 4 : 0u;
+    uint32_t excl = 0, spins = 0, nap = 32;
     const uint32_t limit = spin_limit ? spin_limit : kSpinLimit;
-    while (p >= 0) {
-        W s[kWindow];
+    int32_t p = active ? (int32_t)part - 1 : -1;
+    while (__any_sync(0xffffffffu, p >= 0)) {
+        uint32_t st[kWindow];
+        const int32_t q = p - (int32_t)slot * kWindow;
 #pragma unroll
         for (int w = 0; w < kWindow; ++w)
-            s[w] = (p - w >= 0) ? ld_status(stat + (size_t)(p - w) * stride) : flag_prefix;
-        int used = 0;
-        bool found = false;
-        for (; used < kWindow; ++used) {
-            const W flag = s[used] & ~value_mask;
-            if (flag == 0) break;
-            excl += s[used] & value_mask;
-            if (flag == flag_prefix) {
-                found = true;
-                break;
+            st[w] = (p >= 0 && q - w >= 0) ? ld_relaxed(stat + (size_t)(q - w) * stride) : kFlagPrefix;
+        uint32_t sum = 0, used = 0;
+        bool open = true, found = false;
+#pragma unroll
+        for (int w = 0; w < kWindow; ++w) {
+            open = open && (st[w] & ~kCountMask) != 0;
+            if (open) {
+                sum += st[w] & kCountMask;
+                ++used;
+                found = (st[w] & ~kCountMask) == kFlagPrefix;
+                open = !found;
             }
         }
-        if (found) break;
-        if (used == 0) {
+        if (LPD == 2) {
+            const uint32_t osum = __shfl_xor_sync(0xffffffffu, sum, 16);
+            const uint32_t oused = __shfl_xor_sync(0xffffffffu, used, 16);
+            const bool ofound = __shfl_xor_sync(0xffffffffu, (uint32_t)found, 16) != 0;
+            const uint32_t s0 = slot ? osum : sum, s1 = slot ? sum : osum;
+            const uint32_t u0 = slot ? oused : used, u1 = slot ? used : oused;
+            const bool f0 = slot ? ofound : found, f1 = slot ? found : ofound;
+            const bool both = !f0 && u0 == kWindow;
+            sum = s0 + (both ? s1 : 0u);
+            used = u0 + (both ? u1 : 0u);
+            found = f0 || (both && f1);
+        }
+        if (p >= 0) {
+            excl += sum;
+            p -= (int32_t)used;
+            if (found) p = -1;
+        }
+        if (p >= 0 && used == 0) {
             if (++spins > limit) {
                 atomicOr(err, SF_DEV_ERR_TIMEOUT);
-                break;
+                p = -1;
+            } else {
+                __nanosleep(nap);
+                nap = min(nap * 2u, 256u);
             }
-            __nanosleep(nap);
-            nap = min(nap * 2u, 256u);
         }
-        p -= used;
     }
     return excl;
 }
@@ -133,23 +152,6 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
     return m;
-}
-
-// Lanes holding the same BITS-bit digit (and the same validity) as this
-// lane: one ballot per digit bit, inverted where this lane's bit is clear,
-// ANDed. Fixed cost of BITS + 1 votes, far cheaper on this part than
-// match.any.
-template <int BITS>
-__device__ __forceinline__ uint32_t match_digit(uint32_t d, bool valid) {
-    uint32_t peers = __ballot_sync(0xffffffffu, valid);
-    if (!valid) peers = ~peers;
-#pragma unroll
-    for (int b = 0; b < BITS; ++b) {
-        const bool bit = (d >> b) & 1u;
-        const uint32_t v = __ballot_sync(0xffffffffu, bit);
-        peers &= bit ? v : ~v;
-    }
-    return peers;
 }
 
 __device__ __forceinline__ uint32_t load_n(const uint32_t* n_dev, uint32_t n_static) {
@@ -206,6 +208,202 @@ __global__ __launch_bounds__(kThreads) void radix_histogram_kernel(
         if (s_hist[i]) atomicAdd(&hist[i], s_hist[i]);
 }
 
+// The same counts from kWideHistN keys on. A shared atomic costs a cycle per
+// lane on the busiest bank, so with one counter per bin the random digits of a
+// warp serialise about four deep and four digits per key took 62 us for 10M
+// keys. Here lane l counts in column l of a 32-column table (bank l whatever
+// the digit, equal digits of a warp included): 24 us. The table
+// (up to 128 KB) allows one CTA of 1024 threads per SM, and clearing and
+// summing it costs about 3 us, so smaller inputs keep the form above.
+constexpr uint32_t kWideHistN = 1u << 20;
+constexpr int kWideHistThreads = 1024;
+template <int BITS>
+__global__ __launch_bounds__(kWideHistThreads, 1) void radix_histogram_wide_kernel(
+    const uint32_t* __restrict__ keys, const uint32_t* n_dev, uint32_t n_static, uint32_t num_passes, uint32_t bits,
+    uint32_t* __restrict__ hist) {
+    constexpr uint32_t R = 1u << BITS;
+    constexpr int kLoads = 8;
+    extern __shared__ __align__(16) uint32_t s_cols[];
+    const uint32_t n = load_n(n_dev, n_static);
+    const uint32_t bins = num_passes * R, tid = threadIdx.x, lane = tid & 31u;
+    for (uint32_t i = tid; i < bins * 8; i += kWideHistThreads)
+        reinterpret_cast<uint4*>(s_cols)[i] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+    const uint32_t last_mask = (1u << (bits - (num_passes - 1) * BITS)) - 1u;
+    const uint32_t warps = (gridDim.x * kWideHistThreads) >> 5;
+    for (uint64_t base = (uint64_t)((blockIdx.x * kWideHistThreads + tid) >> 5) * (32 * kLoads); base < n;
+         base += (uint64_t)warps * (32 * kLoads)) {
+        uint32_t kk[kLoads];
+#pragma unroll
+        for (int u = 0; u < kLoads; ++u) {
+            const uint64_t i = base + u * 32 + lane;
+            kk[u] = i < n ? __ldg(keys + i) : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < kLoads; ++u) {
+            if (base + u * 32 + lane >= n) continue;
+            for (uint32_t p = 0; p < num_passes; ++p) {
+                const uint32_t d = (kk[u] >> (p * BITS)) & (p + 1 < num_passes ? R - 1u : last_mask);
+                atomicAdd(&s_cols[(p * R + d) * 32 + lane], 1u);
+            }
+        }
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < bins; i += kWideHistThreads) {
+        uint32_t sum = 0;
+#pragma unroll
+        for (uint32_t c = 0; c < 32; ++c) sum += s_cols[i * 32 + ((c + lane) & 31u)];
+        if (sum) atomicAdd(&hist[i], sum);
+    }
+}
+
+// Shared memory of one digit pass.
+template <int BITS, int THREADS>
+struct PassShared {
+    static constexpr uint32_t R = 1u << BITS;
+    uint32_t keys[THREADS * kItems], vals[THREADS * kItems];  // staged for the scatter
+    // Per warp and digit: the lanes of the item being ranked that hold the
+    // digit; the warp's keys of it so far, later the first staged slot of the
+    // warp's keys of it.
+    uint32_t lanes[THREADS / 32][R], warp[THREADS / 32][R];
+    uint32_t base[R], gstart[R], total[R];
+    uint32_t scan[THREADS / 32];
+    uint32_t part;
+};
+
+// Exclusive prefix of v over the block's threads (two barriers; s_scan is
+// free again after the caller's next barrier).
+template <int THREADS>
+__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t* s_scan) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += t;
+    }
+    __syncthreads();
+    if (lane == 31) s_scan[warp] = incl;
+    __syncthreads();
+    const uint32_t before = lane < warp ? s_scan[lane] : 0u;  // warp < 32
+    return incl - v + __reduce_add_sync(0xffffffffu, before);
+}
+
+// One partition of a digit pass; FULL: all THREADS x kItems keys exist.
+template <int BITS, int THREADS, bool FULL>
+__device__ __forceinline__ void onesweep_partition(
+    PassShared<BITS, THREADS>& sm, const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
+    uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n, uint32_t part, uint32_t shift,
+    uint32_t digit_mask, const uint32_t* __restrict__ pass_hist, uint32_t* lookback, uint32_t* err, int vals_iota,
+    int write_keys, LookbackKnobs knobs) {
+    constexpr uint32_t R = 1u << BITS;
+    constexpr int kPassWarps = THREADS / 32, kPassTile = THREADS * kItems;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t base = part * kPassTile;
+    const uint32_t w0 = base + warp * (kItems * 32) + lane;  // this lane's item i is w0 + 32 i
+
+    uint32_t k[kItems];
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) k[i] = FULL || w0 + i * 32 < n ? keys_in[w0 + i * 32] : 0u;
+    // Stable warp ranking, items in index order, lanes in lane order: each
+    // lane sets its bit in its digit's lane mask; the mask gives its rank
+    // among the item's equal digits, and the first lane of a digit adds them
+    // to the warp's count and clears the mask. Against one ballot per digit
+    // bit (8 votes and 24 more instructions an item), which left the pass
+    // bound by issue slots, this one is bound by shared-memory bank conflicts
+    // (LSU pipe 69% busy, issue 35%): a pass over 10M pairs 84 -> 70 us. With
+    // 6, 10 or all 16 of a thread's items ranked by ballots instead, the
+    // 10M-key sort took 0.315, 0.336 and 0.361 ms against 0.313. rank < 512 (a
+    // warp's keys): two to a word.
+    const uint32_t lt = lanemask_lt(), me = 1u << lane;
+    uint32_t rank[kItems / 2];
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+        const bool valid = FULL || w0 + i * 32 < n;
+        const uint32_t d = (k[i] >> shift) & digit_mask;
+        uint32_t *count = &sm.warp[warp][d], *lanes = &sm.lanes[warp][d];
+        if (valid) atomicOr(lanes, me);
+        __syncwarp();
+        const uint32_t m = *lanes, before = *count;
+        __syncwarp();
+        if (valid && (m & lt) == 0) {
+            *lanes = 0u;
+            *count = before + (uint32_t)__popc(m);
+        }
+        const uint32_t r = before + (uint32_t)__popc(m & lt);
+        rank[i / 2] = i % 2 == 0 ? r : rank[i / 2] | (r << 16);
+        __syncwarp();
+    }
+    __syncthreads();
+
+    // Per digit: the block's count, published; the first staged slot of each
+    // warp's keys of it; the digit's first global slot.
+    uint32_t digit_total = 0;
+    if (tid < R) {
+#pragma unroll
+        for (int w = 0; w < kPassWarps; ++w) digit_total += sm.warp[w][tid];
+        if (part > 0 || !knobs.withhold)
+            st_relaxed(&lookback[(size_t)part * R + tid], (part == 0 ? kFlagPrefix : kFlagAgg) | digit_total);
+    }
+    const uint32_t local = block_exclusive<THREADS>(digit_total, sm.scan);
+    const uint32_t global = block_exclusive<THREADS>(tid < R ? pass_hist[tid] : 0u, sm.scan);
+    if (tid < R) {
+        uint32_t run = local;
+#pragma unroll
+        for (int w = 0; w < kPassWarps; ++w) {
+            const uint32_t c = sm.warp[w][tid];
+            sm.warp[w][tid] = run;
+            run += c;
+        }
+        sm.total[tid] = digit_total;
+        sm.gstart[tid] = global - local;
+    }
+    __syncthreads();
+    // Into shared memory in the partition's sorted order, which needs no
+    // global offset: keys, then values, leave their registers before the
+    // look-back (with both held through it the compiler spilled 36 words).
+    // The digits are formed anew (the empty asm hides that they were known):
+    // sixteen kept slot addresses would be spilled.
+    uint32_t shift2 = shift;
+    asm volatile("" : "+r"(shift2));
+#pragma unroll
+    for (int i = 0; i < kItems; ++i) {
+        if (FULL || w0 + i * 32 < n) {
+            const uint32_t pos = sm.warp[warp][(k[i] >> shift2) & digit_mask] + ((rank[i / 2] >> (i % 2 * 16)) & 0xffffu);
+            sm.keys[pos] = k[i];
+            k[i] = pos;
+        }
+    }
+    uint32_t v[kItems];
+#pragma unroll
+    for (int i = 0; i < kItems; ++i)
+        v[i] = vals_iota ? w0 + i * 32 : (FULL || w0 + i * 32 < n ? vals_in[w0 + i * 32] : 0u);
+#pragma unroll
+    for (int i = 0; i < kItems; ++i)
+        if (FULL || w0 + i * 32 < n) sm.vals[k[i]] = v[i];
+    {
+        constexpr int LPD = THREADS >= 2 * (int)R ? 2 : 1;
+        const uint32_t d = LPD == 2 ? warp * 16 + (lane & 15u) : tid;
+        const bool active = d < R;
+        uint32_t* stat = lookback + (active ? d : 0u);
+        const uint32_t excl = lookback_digit<LPD>(stat, R, part, active, err, knobs.spin_limit);
+        if (active && (LPD == 1 || lane < 16)) {
+            if (part > 0) st_relaxed(&stat[(size_t)part * R], kFlagPrefix | ((excl + sm.total[d]) & kCountMask));
+            sm.base[d] = sm.gstart[d] + excl;
+        }
+    }
+    __syncthreads();
+    const uint32_t cnt = FULL ? (uint32_t)kPassTile : n - base;
+#pragma unroll 4
+    for (uint32_t j = tid; j < cnt; j += THREADS) {
+        const uint32_t key = sm.keys[j];
+        const uint32_t out = sm.base[(key >> shift) & digit_mask] + j;
+        if (out >= n) continue;  // only after a timed-out look-back
+        if (write_keys) keys_out[out] = key;
+        vals_out[out] = sm.vals[j];
+    }
+}
+
 // One BITS-bit digit pass. `vals_iota` substitutes vals_in[i] = i.
 template <int BITS, int THREADS>
 __global__ __launch_bounds__(THREADS, THREADS >= 512 ? 2 : 4) void onesweep_pass_kernel(
@@ -214,150 +412,24 @@ __global__ __launch_bounds__(THREADS, THREADS >= 512 ? 2 : 4) void onesweep_pass
     uint32_t n_static, uint32_t shift, uint32_t digit_mask, const uint32_t* __restrict__ pass_hist,
     uint32_t* lookback, uint32_t* ticket, uint32_t* err, int vals_iota, int write_keys, LookbackKnobs knobs) {
     constexpr uint32_t R = 1u << BITS;
-    constexpr int kPassThreads = THREADS, kPassWarps = THREADS / 32, kPassTile = THREADS * kItems;
-    __shared__ uint32_t s_part;
-    __shared__ uint32_t s_warp_hist[kPassWarps][R];
-    __shared__ uint32_t s_local_start[R];
-    __shared__ uint32_t s_global_base[R];
-    __shared__ uint32_t s_scan[kPassWarps];
-    extern __shared__ __align__(16) uint32_t s_stage[];
-    uint32_t* s_keys = s_stage;
-    uint32_t* s_vals = s_stage + kPassTile;
-
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    constexpr int kPassTile = THREADS * kItems;
+    static_assert(THREADS >= (int)R, "one thread per digit");
+    extern __shared__ __align__(16) unsigned char s_pass[];
+    PassShared<BITS, THREADS>& sm = *reinterpret_cast<PassShared<BITS, THREADS>*>(s_pass);
+    const uint32_t tid = threadIdx.x;
     const uint32_t n = load_n(n_dev, n_static);
     const uint32_t num_parts = (n + kPassTile - 1) / kPassTile;
-    if (tid == 0) s_part = atomicAdd(ticket, 1u);
-    for (uint32_t i = tid; i < kPassWarps * R; i += kPassThreads) (&s_warp_hist[0][0])[i] = 0;
+    if (tid == 0) sm.part = atomicAdd(ticket, 1u);
+    for (uint32_t i = tid; i < THREADS / 32 * R; i += THREADS) (&sm.warp[0][0])[i] = (&sm.lanes[0][0])[i] = 0u;
     __syncthreads();
-    const uint32_t part = s_part;
+    const uint32_t part = sm.part;
     if (part >= num_parts) return;
-    const uint32_t base = part * kPassTile;
-    const uint32_t wbase = base + warp * (kItems * 32);
-
-    // Keys and values are loaded together, before the ranking and the
-    // look-back, so no global load waits behind them.
-    uint32_t k[kItems], rank[kItems], vv[kItems];
-#pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        const uint32_t idx = wbase + i * 32 + lane;
-        k[i] = idx < n ? keys_in[idx] : 0u;
-        vv[i] = idx < n ? (vals_iota ? idx : vals_in[idx]) : 0u;
-    }
-    // Stable warp ranking: items in index order, lanes in lane order.
-    const uint32_t lt = lanemask_lt();
-#pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        const uint32_t idx = wbase + i * 32 + lane;
-        const bool valid = idx < n;
-        const uint32_t d = valid ? ((k[i] >> shift) & digit_mask) : R;
-        const uint32_t peers = match_digit<BITS>(d, valid);
-        const uint32_t leader = __ffs(peers) - 1;
-        uint32_t prev = 0;
-        if (valid && lane == leader) {
-            prev = s_warp_hist[warp][d];
-            s_warp_hist[warp][d] = prev + __popc(peers);
-        }
-        prev = __shfl_sync(0xffffffffu, prev, leader);
-        rank[i] = prev + __popc(peers & lt);
-        __syncwarp();
-    }
-    __syncthreads();
-
-    // Per digit: exclusive prefix over warps, block total, publish.
-    uint32_t digit_total = 0;
-    if (tid < R) {
-        uint32_t sum = 0;
-#pragma unroll
-        for (int w = 0; w < kPassWarps; ++w) {
-            const uint32_t c = s_warp_hist[w][tid];
-            s_warp_hist[w][tid] = sum;
-            sum += c;
-        }
-        digit_total = sum;
-        if (part > 0 || !knobs.withhold)
-            st_relaxed(&lookback[(size_t)part * R + tid], (part == 0 ? kFlagPrefix : kFlagAgg) | sum);
-    }
-    // Block exclusive scan of digit totals (digit order) -> local starts.
-    {
-        uint32_t v = digit_total;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= (uint32_t)o) v += t;
-        }
-        if (lane == 31) s_scan[warp] = v;
-        __syncthreads();
-        if (tid < 32) {
-            uint32_t w = tid < (uint32_t)kPassWarps ? s_scan[tid] : 0u;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= (uint32_t)o) w += t;
-            }
-            if (tid < (uint32_t)kPassWarps) s_scan[tid] = w;
-        }
-        __syncthreads();
-        if (tid < R) s_local_start[tid] = v - digit_total + (warp ? s_scan[warp - 1] : 0u);
-    }
-    // Global digit offsets of this pass (exclusive over digits of pass_hist).
-    uint32_t gstart = 0;
-    {
-        const uint32_t h = tid < R ? pass_hist[tid] : 0u;
-        uint32_t v = h;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, v, o);
-            if (lane >= (uint32_t)o) v += t;
-        }
-        __syncthreads();
-        if (lane == 31) s_scan[warp] = v;
-        __syncthreads();
-        if (tid < 32) {
-            uint32_t w = tid < (uint32_t)kPassWarps ? s_scan[tid] : 0u;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, w, o);
-                if (lane >= (uint32_t)o) w += t;
-            }
-            if (tid < (uint32_t)kPassWarps) s_scan[tid] = w;
-        }
-        __syncthreads();
-        gstart = v - h + (warp ? s_scan[warp - 1] : 0u);
-    }
-    // Decoupled look-back, one digit per thread, kWindow predecessors per step.
-    if (tid < R) {
-        uint32_t excl = 0;
-        if (part > 0) {
-            excl = lookback_window<uint32_t>(lookback + tid, R, part, kFlagPrefix, kCountMask, err,
-                                            knobs.spin_limit);
-            st_relaxed(&lookback[(size_t)part * R + tid], kFlagPrefix | ((excl + digit_total) & kCountMask));
-        }
-        s_global_base[tid] = gstart + excl - s_local_start[tid];
-    }
-    __syncthreads();
-
-    // Scatter into shared memory at the partition-local sorted position.
-#pragma unroll
-    for (int i = 0; i < kItems; ++i) {
-        const uint32_t idx = wbase + i * 32 + lane;
-        if (idx < n) {
-            const uint32_t d = (k[i] >> shift) & digit_mask;
-            const uint32_t pos = s_local_start[d] + s_warp_hist[warp][d] + rank[i];
-            s_keys[pos] = k[i];
-            s_vals[pos] = vv[i];
-        }
-    }
-    __syncthreads();
-    const uint32_t cnt = min((uint32_t)kPassTile, n - base);
-    for (uint32_t j = tid; j < cnt; j += kPassThreads) {
-        const uint32_t key = s_keys[j];
-        const uint32_t d = (key >> shift) & digit_mask;
-        const uint32_t out = s_global_base[d] + j;
-        if (out >= n) continue;  // only after a timed-out look-back
-        if (write_keys) keys_out[out] = key;
-        vals_out[out] = s_vals[j];
-    }
+    if (n - part * kPassTile >= (uint32_t)kPassTile)
+        onesweep_partition<BITS, THREADS, true>(sm, keys_in, vals_in, keys_out, vals_out, n, part, shift, digit_mask,
+                                                pass_hist, lookback, err, vals_iota, write_keys, knobs);
+    else
+        onesweep_partition<BITS, THREADS, false>(sm, keys_in, vals_in, keys_out, vals_out, n, part, shift,
+                                                 digit_mask, pass_hist, lookback, err, vals_iota, write_keys, knobs);
 }
 
 // The scan's look-back done by one whole warp: lane l reads the status of
@@ -366,7 +438,7 @@ __global__ __launch_bounds__(THREADS, THREADS >= 512 ? 2 : 4) void onesweep_pass
 // every lane before it an aggregate, the warp sums those lanes and stops;
 // otherwise it sums the aggregates before the first lane whose partition
 // has published nothing and reads again from there, with the same backoff
-// and bound as lookback_window. Lanes past partition 0 read a zero prefix.
+// and bound as lookback_digit. Lanes past partition 0 read a zero prefix.
 // Returns the exclusive prefix in every lane.
 __device__ unsigned long long lookback_warp64(const unsigned long long* stat, uint32_t part, uint32_t* err,
                                               uint32_t spin_limit, unsigned long long flag_prefix,
@@ -533,15 +605,24 @@ cudaError_t radix_sort_bits(const uint32_t* keys_in, const uint32_t* vals_in, ui
     cudaError_t e = cudaMemsetAsync(temp, 0, kHistWords * 4 + 64 + passes * parts * R * 4, stream);
     if (e != cudaSuccess) return e;
     if (parts == 0) { *out_in_b = 0; return cudaSuccess; }
-    const uint32_t hist_blocks = (uint32_t)std::min<size_t>((grid_n + kThreads * 8 - 1) / (kThreads * 8),
-                                                             (size_t)sm_count * 4);
-    radix_histogram_kernel<BITS><<<std::max(hist_blocks, 1u), kThreads, 0, stream>>>(
-        keys_in, n_dev, n, passes, bits, hist);
+    if (grid_n >= kWideHistN) {
+        const size_t smem = (size_t)passes * R * 32 * 4;
+        e = cudaFuncSetAttribute(radix_histogram_wide_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem);
+        if (e != cudaSuccess) return e;
+        radix_histogram_wide_kernel<BITS><<<(uint32_t)std::max(sm_count, 1), kWideHistThreads, smem, stream>>>(
+            keys_in, n_dev, n, passes, bits, hist);
+    } else {
+        const uint32_t hist_blocks = (uint32_t)std::min<size_t>((grid_n + kThreads * 8 - 1) / (kThreads * 8),
+                                                                 (size_t)sm_count * 4);
+        radix_histogram_kernel<BITS><<<std::max(hist_blocks, 1u), kThreads, 0, stream>>>(
+            keys_in, n_dev, n, passes, bits, hist);
+    }
     int in_b = 0;
     auto run_passes = [&](auto threads) -> cudaError_t {
         constexpr int TH = decltype(threads)::value;
         cudaError_t e2 = cudaFuncSetAttribute(onesweep_pass_kernel<BITS, TH>,
-                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pass_smem<TH>());
+                                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PassShared<BITS, TH>));
         if (e2 != cudaSuccess) return e2;
         const uint32_t* kin = keys_in;
         const uint32_t* vin = vals_in;
@@ -551,7 +632,7 @@ cudaError_t radix_sort_bits(const uint32_t* keys_in, const uint32_t* vals_in, ui
             uint32_t* kout = (p % 2 == 0) ? keys_a : keys_b;
             uint32_t* vout = (p % 2 == 0) ? vals_a : vals_b;
             const bool wk = write_keys || (p + 1 < passes);
-            onesweep_pass_kernel<BITS, TH><<<(uint32_t)parts, TH, pass_smem<TH>(), stream>>>(
+            onesweep_pass_kernel<BITS, TH><<<(uint32_t)parts, TH, sizeof(PassShared<BITS, TH>), stream>>>(
                 kin, vin, kout, vout, n_dev, n, shift, (1u << w) - 1u, hist + p * R,
                 lookback + (size_t)p * parts * R, tickets + p, err, (vals_iota && p == 0) ? 1 : 0,
                 wk ? 1 : 0, knobs);
