@@ -1336,7 +1336,7 @@ int sf_render_backward(sf_splats s, sf_scratch scratch, const sf_camera* cam, ui
         SF_CK(launch_raster_bwd(a, st));
         sf_view view;
         view_for_camera(*cam, w, h, &view);
-        SF_CK(launch_project_bwd(view, s->attr, s->sh, s->n, s->K, d2d, d_attr, d_sh, st));
+        SF_CK(launch_project_bwd(view, s->attr, s->sh, s->n, s->K, scratch->color, d2d, d_attr, d_sh, st));
         return SF_OK;
     })
 }

@@ -266,18 +266,39 @@ __global__ __launch_bounds__(kBwdThreads, 4) void raster_bwd_kernel(BwdArgs a) {
 struct V3 { float x, y, z; };
 __device__ __forceinline__ float dot3(V3 a, V3 b) { return (a.x * b.x + a.y * b.y) + a.z * b.z; }
 
+// One thread per splat; bound by HBM (K = 16: 44 + 36 bytes read, 236 written
+// and up to 192 of SH read per splat). The block's 2D adjoints are one
+// contiguous run, copied to shared memory in whole lines (a thread's nine words
+// lie 36 bytes apart from the next one's). The SH planes are read only for
+// splats with a colour adjoint (7 to 33% of them contribute to a
+// frame), all at once before their first use: with none, their sum into the
+// direction's gradient is zero, unless a coefficient is not finite, which
+// shows in the forward's colour. 1M splats, K = 16: 163 -> 116 us (reading
+// every plane, 36-byte strides); held to 96 or 80 registers the coefficients
+// spill.
+constexpr uint32_t kProjBwdThreads = 128;
 template <int K>
-__global__ __launch_bounds__(256) void project_bwd_kernel(sf_view v, const float* __restrict__ attr,
-                                                          const float* __restrict__ shs, uint32_t n,
-                                                          const float* __restrict__ d2d,
-                                                          float* __restrict__ d_attr,
-                                                          float* __restrict__ d_sh) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+__global__ __launch_bounds__(kProjBwdThreads) void project_bwd_kernel(sf_view v, const float* __restrict__ attr,
+                                                                      const float* __restrict__ shs, uint32_t n,
+                                                                      const float4* __restrict__ color,
+                                                                      const float* __restrict__ d2d,
+                                                                      float* __restrict__ d_attr,
+                                                                      float* __restrict__ d_sh) {
+    __shared__ float s_d2d[kProjBwdThreads * 9];
+    const uint32_t i0 = blockIdx.x * kProjBwdThreads;
+    const uint32_t i = i0 + threadIdx.x;
     const size_t N = n;
+    const uint32_t words = min(kProjBwdThreads, n - i0) * 9u;
+    for (uint32_t q = threadIdx.x; q < words; q += kProjBwdThreads) s_d2d[q] = __ldg(d2d + (size_t)i0 * 9 + q);
     float a[11];
+    float4 col = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (i < n) {
 #pragma unroll
-    for (int k = 0; k < 11; ++k) a[k] = __ldg(attr + k * N + i);
+        for (int k = 0; k < 11; ++k) a[k] = __ldg(attr + k * N + i);
+        col = __ldg(color + i);
+    }
+    __syncthreads();
+    if (i >= n) return;
     const float opacity = sigmoid_(a[10]);
     const V3 mean{a[0], a[1], a[2]};
     const V3 rot0{v.rot0[0], v.rot0[1], v.rot0[2]};
@@ -293,7 +314,13 @@ __global__ __launch_bounds__(256) void project_bwd_kernel(sf_view v, const float
     }
     float g[9];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) g[k] = d2d[(size_t)i * 9 + k];
+    for (int k = 0; k < 9; ++k) g[k] = s_d2d[threadIdx.x * 9 + k];
+    // Whether the SH sum below can be anything but zero.
+    const float reach = (fabsf(col.x) + fabsf(col.y)) + fabsf(col.z);
+    const bool want_sh = g[5] != 0.0f || g[6] != 0.0f || g[7] != 0.0f || !(reach < INFINITY);
+    float c_sh[3 * K];
+#pragma unroll
+    for (int k = 0; k < 3 * K; ++k) c_sh[k] = want_sh ? __ldg(shs + k * N + i) : 0.0f;
     const float cam_x = dot3(rot0, mean) + v.trans[0];
     const float cam_y = dot3(rot1, mean) + v.trans[1];
     const float qw = a[3], qx = a[4], qy = a[5], qz = a[6];
@@ -379,7 +406,7 @@ __global__ __launch_bounds__(256) void project_bwd_kernel(sf_view v, const float
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
             d_sh[(size_t)(k * 3 + c) * N + i] = g[5 + c] * B[k];
-            wsum += g[5 + c] * __ldg(shs + (size_t)(k * 3 + c) * N + i);
+            wsum += g[5 + c] * c_sh[k * 3 + c];
         }
         ddir[0] += wsum * dB[k][0];
         ddir[1] += wsum * dB[k][1];
@@ -479,10 +506,10 @@ cudaError_t launch_raster_bwd(const BwdArgs& a, cudaStream_t stream) {
 }
 
 cudaError_t launch_project_bwd(const sf_view& view, const float* attr, const float* sh, uint32_t n,
-                               uint32_t sh_per_ch, const float* d2d, float* d_attr, float* d_sh,
-                               cudaStream_t stream) {
+                               uint32_t sh_per_ch, const float4* color, const float* d2d, float* d_attr,
+                               float* d_sh, cudaStream_t stream) {
     if (n == 0) return cudaSuccess;
-    const uint32_t grid = (n + 255) / 256;
+    const uint32_t grid = (n + kProjBwdThreads - 1) / kProjBwdThreads;
     // Coefficients past the largest whole SH degree are never read by the
     // forward (the reference's `chs >= 4/9/16` tests): zero gradient.
     const uint32_t used = sh_degree_coeffs(sh_per_ch);
@@ -492,10 +519,15 @@ cudaError_t launch_project_bwd(const sf_view& view, const float* attr, const flo
         if (e != cudaSuccess) return e;
     }
     switch (used) {
-        case 1: project_bwd_kernel<1><<<grid, 256, 0, stream>>>(view, attr, sh, n, d2d, d_attr, d_sh); break;
-        case 4: project_bwd_kernel<4><<<grid, 256, 0, stream>>>(view, attr, sh, n, d2d, d_attr, d_sh); break;
-        case 9: project_bwd_kernel<9><<<grid, 256, 0, stream>>>(view, attr, sh, n, d2d, d_attr, d_sh); break;
-        case 16: project_bwd_kernel<16><<<grid, 256, 0, stream>>>(view, attr, sh, n, d2d, d_attr, d_sh); break;
+#define SF_PROJECT_BWD(K)                                                                                       \
+    case K:                                                                                                     \
+        project_bwd_kernel<K><<<grid, kProjBwdThreads, 0, stream>>>(view, attr, sh, n, color, d2d, d_attr, d_sh); \
+        break;
+        SF_PROJECT_BWD(1)
+        SF_PROJECT_BWD(4)
+        SF_PROJECT_BWD(9)
+        SF_PROJECT_BWD(16)
+#undef SF_PROJECT_BWD
         default: return cudaErrorInvalidValue;
     }
     note_launches(1);

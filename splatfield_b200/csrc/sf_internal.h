@@ -150,8 +150,8 @@ struct BwdArgs {
 };
 cudaError_t launch_raster_bwd(const BwdArgs& a, cudaStream_t stream);
 cudaError_t launch_project_bwd(const sf_view& view, const float* attr, const float* sh, uint32_t n,
-                               uint32_t sh_per_ch, const float* d2d, float* d_attr, float* d_sh,
-                               cudaStream_t stream);
+                               uint32_t sh_per_ch, const float4* color, const float* d2d, float* d_attr,
+                               float* d_sh, cudaStream_t stream);
 
 // Reference-layout projected rows [n][9] from the split records.
 cudaError_t launch_export_rows(const float4* geo0, const float4* geo1, const float4* color,
