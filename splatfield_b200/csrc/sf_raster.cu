@@ -18,11 +18,22 @@
 // saturation count) before compositing it.
 //
 // Per pair: the power of the splat's quadratic form at the pixel; a pair with
-// power above the splat's power_max (alpha < 1/255 for sure) skips the
-// exponential; alpha = min(opacity * exp(-power), 0.999), pairs below 1/255
-// are skipped, and the pixel stops after the contributor that takes T below
-// 1/255 (src/raster.rs:173-221). The f32 operations are the oracle's, in the
-// same order (sf_math.cuh), so images and words are bit-identical to it.
+// power above the splat's power_max (alpha < 1/255 for sure) is skipped;
+// alpha = min(opacity * exp(-power), 0.999), pairs below 1/255 are skipped,
+// and the pixel stops after the contributor that takes T below 1/255
+// (src/raster.rs:173-221). The f32 operations are the oracle's, in the same
+// order (sf_math.cuh), so images and words are bit-identical to it.
+//
+// What bounds the walk is instruction issue (about 65% of the slots at 1080p,
+// the rest barriers and the tail of long tiles), so it takes two entries at a
+// time: a warp packs the entries it walks into pair records (PairRec), and the
+// two powers and exponentials are one chain of packed f32 operations, which
+// round each half as the scalar ones do. Only the composite itself stays in
+// list order, and it is written with predicates. 1M splats at 1080p: 178 ->
+// 160 us and 127M -> 108M warp instructions against packed pairs with branches
+// in the composite, and 190 us with one entry at a time; 3001 splats at 97x61,
+// where the chain's latency counts, 43 -> 27 us. A limit of 48 registers (five
+// CTAs an SM instead of four) spilled 12 words and took 173 us.
 //
 // CULL: each warp walks only the entries that can reach its 8x4 block (the
 // power_max box from the projection, then the exact test of sf_tile.cuh), 32
@@ -87,6 +98,68 @@ struct ModeOf {
     static constexpr bool kReal = MODE == 3;
 };
 
+// Two consecutive list entries a and b of a warp's walk, each field of both
+// side by side, so that one 16-byte load fills the operands of two packed f32
+// operations: centres, negated form coefficients and power_max, opacity, the
+// entries' places in the staged chunk and (RGB) colours. The stride (80 or 112
+// bytes) starts the 16 records of a warp in eight different banks.
+template <bool COLOR>
+struct __align__(16) PairRec {
+    float x[2], y[2], nhx[2], ncy[2], nhz[2], op[2], npm[2];
+    uint32_t j[2];
+    float r[COLOR ? 2 : 1], g[COLOR ? 2 : 1], b[COLOR ? 2 : 1];
+    uint32_t pad[COLOR ? 6 : 1];
+};
+static_assert(sizeof(PairRec<true>) == 112 && sizeof(PairRec<false>) == 80, "record stride");
+
+// Packed f32 pairs (sm_100a): each half rounds as the scalar operation does.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 both(float v) { return pack2(v, v); }
+
+// exp_neg_ (sf_math.cuh) of two values, operation by operation.
+__device__ __forceinline__ void exp_neg2(f32x2 x, float& ea, float& eb) {
+    const f32x2 kr = add2(mul2(x, both(1.44269502f)), both(12582912.0f));
+    const f32x2 kf = add2(kr, both(-12582912.0f));
+    f32x2 r = fma2(kf, both(-0.693145751953125f), x);
+    r = fma2(kf, both(-1.42860677e-06f), r);
+    f32x2 p = both(1.98412701e-04f);
+    p = fma2(p, r, both(1.38888892e-03f));
+    p = fma2(p, r, both(8.33333377e-03f));
+    p = fma2(p, r, both(4.16666679e-02f));
+    p = fma2(p, r, both(1.66666672e-01f));
+    p = fma2(p, r, both(0.5f));
+    p = fma2(p, r, both(1.0f));
+    p = fma2(p, r, both(1.0f));
+    float pa, pb, ka, kb;
+    unpack2(p, pa, pb);
+    unpack2(kr, ka, kb);
+    ea = u2f(f2u(pa) + (f2u(ka) << 23));
+    eb = u2f(f2u(pb) + (f2u(kb) << 23));
+}
+
 // Shared staging of one CTA: two buffers of kChunk records each.
 template <int MODE, bool CULL, uint32_t NT>
 struct Stage {
@@ -98,6 +171,8 @@ struct Stage {
     uint32_t gid[kW || kR ? 2 : 1][kW || kR ? kChunk : 1];
     uint32_t acc0[kW ? 2 : 1][kW ? kChunk : 1];
     uint32_t acc1[MODE == 2 ? 2 : 1][MODE == 2 ? kChunk : 1];
+    // The entries a warp walks next, two by two (PairRec).
+    PairRec<kC> pairs[NT / 32][16];
     // Each warp's sums of the chunk being walked (zero when it is staged).
     float part[kR ? 2 : 1][kR ? NT / 32 : 1][kR ? kChunk : 1];
 };
@@ -105,7 +180,6 @@ struct Stage {
 struct PixelState {
     float T, pr, pg, pb;
     uint32_t last;
-    bool done;
     uint32_t n_eval, n_hit, n_proc;
 };
 
@@ -113,9 +187,10 @@ struct PixelState {
 // gives entry i's splat id, list_off the entry's position in the tile's
 // whole sorted list. (wxf, wyf): the first pixel centre of this warp's 8x4
 // block. Returns true once every pixel of the CTA is saturated (uniform).
-// STATE: ps.last tracks the last contributor (for the adjoint); otherwise
-// only the entry that saturated the pixel.
-template <int MODE, bool CULL, bool DETAIL, bool STATE, uint32_t NT, typename IdOf>
+// EXACT: ps.last is the pixel's last contributor (1-based position); otherwise
+// the end of the chunk it lies in, which is all that the pair statistics need
+// of a list that is walked from its start.
+template <int MODE, bool CULL, bool DETAIL, bool EXACT, uint32_t NT, typename IdOf>
 __device__ bool composite_list(const RasterArgs& a, Stage<MODE, CULL, NT>& sm, IdOf id, uint32_t count,
                                uint32_t list_off, float fx, float fy, float wxf, float wyf, uint32_t inside,
                                PixelState& ps) {
@@ -182,96 +257,171 @@ __device__ bool composite_list(const RasterArgs& a, Stage<MODE, CULL, NT>& sm, I
             }
         }
     };
-    // One (warp, entry) step: every lane of the warp runs it together; returns
-    // this pixel's weight alpha T (mode 3).
-    auto step = [&](uint32_t b, uint32_t j, uint32_t pos) -> float {
-        if (DETAIL) ++ps.n_proc;
-        uint32_t q = 0;
-        float weight = 0.0f;
-        // CULL: a warp whose pixels are all done has left the chunk, so the
-        // power is formed unconditionally and one branch tests both.
-        if (CULL || !ps.done) {
-            const float4 g0 = sm.g0[b][j];
-            const float4 g1 = sm.g1[b][j];
-            const float dx = g0.x - fx, dy = g0.y - fy;
-            const float power = fma_(g0.z * dx, dx, fma_(g1.x * dy, dy, (g0.w * dx) * dy));
-            if ((!CULL || !ps.done) && !(power > g1.z)) {
-                if (DETAIL) ++ps.n_eval;
-                const float alpha = fminf(g1.y * exp_neg_(-power), 0.999f);
-                if (alpha >= inv255) {
-                    if (DETAIL) ++ps.n_hit;
-                    const float vis = alpha * ps.T;
-                    if (kColor) {
-                        const float4 c = sm.col[b][j];
-                        ps.pr = fma_(c.x, vis, ps.pr);
-                        ps.pg = fma_(c.y, vis, ps.pg);
-                        ps.pb = fma_(c.z, vis, ps.pb);
-                    } else if (kWords) {
-                        q = sat_u32(vis * a.scale);
-                    } else if (kReal) {
-                        weight = vis;
-                    }
-                    ps.T = ps.T * (1.0f - alpha);
-                    if (STATE) ps.last = pos;
-                    if (ps.T < inv255) {
-                        ps.done = true;
-                        if (!STATE) ps.last = pos;
-                    }
-                }
-            }
-        }
-        if (kWords) {
-            if (__any_sync(0xffffffffu, q != 0u)) {
-                if (MODE == 1) {
-                    const uint32_t s = __reduce_add_sync(0xffffffffu, q);
-                    if (lane == 0) atomicAdd(&sm.acc0[b][j], s);
-                } else {
-                    const uint32_t qf = inside ? q : 0u;
-                    const uint32_t sf = __reduce_add_sync(0xffffffffu, qf);
-                    const uint32_t st = __reduce_add_sync(0xffffffffu, q);
-                    if (lane == 0) {
-                        if (sf) atomicAdd(&sm.acc0[b][j], sf);
-                        if (st - sf) atomicAdd(&sm.acc1[b][j], st - sf);
-                    }
-                }
-            }
-        }
-        return weight;
-    };
     // Mode 3: whether this warp's pixels lie on both sides of the mask, else
     // which side they are on.
     const bool mixed = kReal && !__all_sync(0xffffffffu, inside) && __any_sync(0xffffffffu, inside);
     const uint32_t side = kReal && inside ? 0u : 1u;
-    // Mode 3: steps over the entries of the ballot word, four at a time.
-    auto step_real = [&](uint32_t b, uint32_t g32, uint32_t word, uint32_t pos0) {
-        while (word) {
-            float v[4];
-            uint32_t mine = 0;  // the entry whose sum this lane ends with
-            const uint32_t which = mixed ? (lane >> 2) & 3u : lane >> 3;
-#pragma unroll
-            for (uint32_t u = 0; u < 4; ++u) {
-                v[u] = 0.0f;
-                if (word) {
-                    const uint32_t jj = g32 + (uint32_t)(__ffs(word) - 1);
-                    word &= word - 1u;
-                    if (which == u) mine = jj;
-                    v[u] = step(b, jj, pos0 + jj);
-                }
+    const f32x2 nfx = both(-fx), nfy = both(-fy);
+    auto* const recs = sm.pairs[warp];
+    auto done = [&]() { return ps.T < inv255; };
+
+    // Composites one entry into this lane's pixel: npow = -power, e =
+    // exp(npow); returns alpha T where the entry contributes (the pixel is not
+    // saturated, T >= 1/255; alpha >= 1/255; power no higher than power_max or
+    // NaN), else 0. Written with predicates: as branches, the two entries of a
+    // pair cost a third more instructions.
+    auto composite = [&](float npow, float npm, float op, float e, float cr, float cg, float cb,
+                         uint32_t pos) -> float {
+        const float alpha = fminf(op * e, 0.999f);
+        float vis;
+        if (DETAIL) {
+            const bool eval = ps.T >= inv255 && !(npow < npm);
+            ps.n_eval += eval;
+            ps.n_hit += eval && alpha >= inv255;
+        }
+        const float t0 = ps.T;
+        if constexpr (kColor) {
+            asm("{\n"
+                ".reg .pred p;\n"
+                ".reg .f32 m;\n"
+                "setp.ge.f32 p, %0, %5;\n"
+                "setp.ge.and.f32 p, %6, %5, p;\n"
+                "setp.geu.and.f32 p, %7, %8, p;\n"
+                "mul.rn.f32 %4, %6, %0;\n"
+                "sub.rn.f32 m, 0f3F800000, %6;\n"
+                "@p fma.rn.f32 %1, %9, %4, %1;\n"
+                "@p fma.rn.f32 %2, %10, %4, %2;\n"
+                "@p fma.rn.f32 %3, %11, %4, %3;\n"
+                "@p mul.rn.f32 %0, %0, m;\n"
+                "}"
+                : "+f"(ps.T), "+f"(ps.pr), "+f"(ps.pg), "+f"(ps.pb), "=&f"(vis)
+                : "f"(inv255), "f"(alpha), "f"(npow), "f"(npm), "f"(cr), "f"(cg), "f"(cb));
+        } else {
+            asm("{\n"
+                ".reg .pred p;\n"
+                ".reg .f32 m;\n"
+                "setp.ge.f32 p, %0, %2;\n"
+                "setp.ge.and.f32 p, %3, %2, p;\n"
+                "setp.geu.and.f32 p, %4, %5, p;\n"
+                "mul.rn.f32 %1, %3, %0;\n"
+                "sub.rn.f32 m, 0f3F800000, %3;\n"
+                "selp.f32 %1, %1, 0f00000000, p;\n"
+                "@p mul.rn.f32 %0, %0, m;\n"
+                "}"
+                : "+f"(ps.T), "=&f"(vis)
+                : "f"(inv255), "f"(alpha), "f"(npow), "f"(npm));
+        }
+        if (EXACT && ps.T != t0) ps.last = pos;  // T always falls where the entry contributes
+        return vis;
+    };
+    // The warp's 32 shares of entry j to its shared accumulators.
+    auto add_words = [&](uint32_t q, uint32_t b, uint32_t j) {
+        if (!__any_sync(0xffffffffu, q != 0u)) return;
+        if (MODE == 1) {
+            const uint32_t s = __reduce_add_sync(0xffffffffu, q);
+            if (lane == 0) atomicAdd(&sm.acc0[b][j], s);
+        } else {
+            const uint32_t qf = inside ? q : 0u;
+            const uint32_t sf = __reduce_add_sync(0xffffffffu, qf);
+            const uint32_t st = __reduce_add_sync(0xffffffffu, q);
+            if (lane == 0) {
+                if (sf) atomicAdd(&sm.acc0[b][j], sf);
+                if (st - sf) atomicAdd(&sm.acc1[b][j], st - sf);
             }
-            const float any = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
-            if (!__any_sync(0xffffffffu, any != 0.0f)) continue;
-            if (mixed) {
-                float x[8];
+        }
+    };
+    // The two entries of recs[p]: both alphas by packed operations, then the
+    // pixel takes them in order. Every lane of the warp runs it together.
+    auto step2 = [&](uint32_t p, uint32_t b, uint32_t pos0, float& wa, float& wb, uint32_t& ja, uint32_t& jb) {
+        const float4* r4 = reinterpret_cast<const float4*>(recs + p);
+        const ulonglong2* r = reinterpret_cast<const ulonglong2*>(recs + p);
+        const ulonglong2 xy = r[0], hc = r[1], zo = r[2];
+        const float4 mj = r4[3];
+        float4 rg = make_float4(0.f, 0.f, 0.f, 0.f);
+        float2 bl = make_float2(0.f, 0.f);
+        if (kColor) {
+            rg = r4[4];
+            bl = *reinterpret_cast<const float2*>(r4 + 5);
+        }
+        ja = f2u(mj.z);
+        jb = f2u(mj.w);
+        const f32x2 dx = add2(xy.x, nfx), dy = add2(xy.y, nfy);
+        const f32x2 npow = fma2(mul2(hc.x, dx), dx, fma2(mul2(zo.x, dy), dy, mul2(mul2(hc.y, dx), dy)));
+        float na, nb, oa, ob, ea, eb;
+        exp_neg2(npow, ea, eb);
+        unpack2(npow, na, nb);
+        unpack2(zo.y, oa, ob);
+        wa = composite(na, mj.x, oa, ea, rg.x, rg.z, bl.x, pos0 + ja);
+        wb = composite(nb, mj.y, ob, eb, rg.y, rg.w, bl.y, pos0 + jb);
+        if (kWords) {
+            add_words(sat_u32(wa * a.scale), b, ja);
+            add_words(sat_u32(wb * a.scale), b, jb);
+        }
+    };
+    // Up to 32 candidates [g32, g32 + 32) of buffer b, of which this lane's is
+    // walked when `hit`: the hits are packed two by two into recs in list
+    // order (an odd last one beside an entry of opacity 0) and composited.
+    auto walk = [&](uint32_t b, uint32_t g32, bool hit, const float4& g0, const float4& g1, uint32_t pos0) {
+        const uint32_t word = __ballot_sync(0xffffffffu, hit);
+        const uint32_t hits = (uint32_t)__popc(word);
+        if (hits == 0) return;
+        if (DETAIL) ps.n_proc += hits;
+        __syncwarp();  // the last group's records have been read
+        if (hit) {
+            const uint32_t slot = (uint32_t)__popc(word & ((1u << lane) - 1u)), h = slot & 1u;
+            auto& r = recs[slot >> 1];
+            if (kColor) {
+                const float4 c = sm.col[b][g32 + lane];
+                r.r[h] = c.x;
+                r.g[h] = c.y;
+                r.b[h] = c.z;
+            }
+            r.x[h] = g0.x;
+            r.y[h] = g0.y;
+            r.nhx[h] = -g0.z;
+            r.ncy[h] = -g0.w;
+            r.nhz[h] = -g1.x;
+            r.op[h] = g1.y;
+            r.npm[h] = -g1.z;
+            r.j[h] = g32 + lane;
+        }
+        if ((hits & 1u) && lane == 0) {
+            auto& r = recs[hits >> 1];
+            r.x[1] = r.y[1] = r.nhx[1] = r.ncy[1] = r.nhz[1] = r.op[1] = r.npm[1] = 0.0f;
+            if (kColor) r.r[1] = r.g[1] = r.b[1] = 0.0f;
+            r.j[1] = g32;
+        }
+        __syncwarp();
+        const uint32_t np = (hits + 1u) >> 1;
+        if constexpr (!kReal) {
+            float wa, wb;
+            uint32_t ja, jb;
+            for (uint32_t p = 0; p < np; ++p) step2(p, b, pos0, wa, wb, ja, jb);
+        } else {
+            // Mode 3: four entries' weights are summed over the warp at once.
+            const uint32_t which = mixed ? (lane >> 2) & 3u : lane >> 3;
+            for (uint32_t p = 0; p < np; p += 2) {
+                float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                uint32_t j[4] = {0u, 0u, 0u, 0u};
+                step2(p, b, pos0, v[0], v[1], j[0], j[1]);
+                if (p + 1 < np) step2(p + 1, b, pos0, v[2], v[3], j[2], j[3]);
+                const float any = fmaxf(fmaxf(v[0], v[1]), fmaxf(v[2], v[3]));
+                if (!__any_sync(0xffffffffu, any != 0.0f)) continue;
+                // The entry whose sum this lane ends with.
+                const uint32_t mine = which < 2 ? (which == 0 ? j[0] : j[1]) : (which == 2 ? j[2] : j[3]);
+                if (mixed) {
+                    float x[8];
 #pragma unroll
-                for (uint32_t u = 0; u < 4; ++u) {
-                    x[u] = inside ? v[u] : 0.0f;
-                    x[4 + u] = inside ? 0.0f : v[u];
+                    for (uint32_t u = 0; u < 4; ++u) {
+                        x[u] = inside ? v[u] : 0.0f;
+                        x[4 + u] = inside ? 0.0f : v[u];
+                    }
+                    warp_sum_scatter(x);
+                    if ((lane & 3u) == 0 && x[0] != 0.0f) sm.part[lane >> 4][warp][mine] = x[0];
+                } else {
+                    warp_sum_scatter(v);
+                    if ((lane & 7u) == 0 && v[0] != 0.0f) sm.part[side][warp][mine] = v[0];
                 }
-                warp_sum_scatter(x);
-                if ((lane & 3u) == 0 && x[0] != 0.0f) sm.part[lane >> 4][warp][mine] = x[0];
-            } else {
-                warp_sum_scatter(v);
-                if ((lane & 7u) == 0 && v[0] != 0.0f) sm.part[side][warp][mine] = v[0];
             }
         }
     };
@@ -292,32 +442,24 @@ __device__ bool composite_list(const RasterArgs& a, Stage<MODE, CULL, NT>& sm, I
         }
         cp_async_commit();
         cp_async_wait<1>();  // this thread's copies of chunk c have landed
-        if (__syncthreads_count(ps.done) == NT) {
+        if (__syncthreads_count(done()) == NT) {
             cp_async_wait<0>();
             return true;
         }
         const uint32_t cnt = min(kChunk, count - c * kChunk);
+        if (!EXACT && !done()) ps.last = c * kChunk + cnt;
         const uint32_t pos0 = list_off + c * kChunk + 1;
-        if (CULL) {
-            for (uint32_t g32 = 0; g32 < cnt; g32 += 32) {
-                if (__all_sync(0xffffffffu, ps.done)) break;
-                const uint32_t j = g32 + lane;
-                const bool hit = j < cnt && block_hit(sm.g0[b][j], sm.g1[b][j], sm.ext[b][j], wxf, wyf);
-                uint32_t word = __ballot_sync(0xffffffffu, hit);
-                if constexpr (kReal) {
-                    step_real(b, g32, word, pos0);
-                }
-                while (!kReal && word) {
-                    const uint32_t jj = g32 + (uint32_t)(__ffs(word) - 1);
-                    word &= word - 1u;
-                    step(b, jj, pos0 + jj);
-                }
+        for (uint32_t g32 = 0; g32 < cnt; g32 += 32) {
+            if (__all_sync(0xffffffffu, done())) break;
+            const uint32_t j = g32 + lane;
+            bool hit = j < cnt;
+            float4 g0 = make_float4(0.f, 0.f, 0.f, 0.f), g1 = g0;
+            if (hit) {
+                g0 = sm.g0[b][j];
+                g1 = sm.g1[b][j];
+                if (CULL) hit = block_hit(g0, g1, sm.ext[b][j], wxf, wyf);
             }
-        } else if (kReal) {
-            for (uint32_t g32 = 0; g32 < cnt; g32 += 32)
-                step_real(b, g32, cnt - g32 < 32 ? (1u << (cnt - g32)) - 1u : 0xffffffffu, pos0);
-        } else {
-            for (uint32_t j = 0; j < cnt; ++j) step(b, j, pos0 + j);
+            walk(b, g32, hit, g0, g1, pos0);
         }
     }
     __syncthreads();
@@ -380,14 +522,26 @@ __device__ void bitonic_sort64(unsigned long long* v, uint32_t m) {
     }
 }
 
+// Shared memory of one CTA.
+template <int MODE, bool CULL, bool LAZY, uint32_t NT>
+struct TileShared {
+    Stage<MODE, CULL, NT> stage;
+    unsigned long long slab[LAZY ? kSlab : 1];
+    unsigned long long s64[16];
+    uint32_t hist[LAZY ? 256 : 1];
+    uint32_t ctl[4];
+};
+
 // This CTA's part `sub` of one tile (block-uniform).
 template <int MODE, bool CULL, bool DETAIL, bool STATE, bool LAZY, uint32_t NT>
 __device__ __forceinline__ void raster_tile(const RasterArgs& a, const uint32_t tile, const uint32_t sub) {
-    __shared__ Stage<MODE, CULL, NT> sm;
-    __shared__ unsigned long long s_slab[LAZY ? kSlab : 1];
-    __shared__ uint32_t s_hist[LAZY ? 256 : 1];
-    __shared__ unsigned long long s_64[16];
-    __shared__ uint32_t s_ctl[4];
+    extern __shared__ __align__(16) unsigned char s_tile[];
+    TileShared<MODE, CULL, LAZY, NT>& sh = *reinterpret_cast<TileShared<MODE, CULL, LAZY, NT>*>(s_tile);
+    Stage<MODE, CULL, NT>& sm = sh.stage;
+    unsigned long long* const s_slab = sh.slab;
+    uint32_t* const s_hist = sh.hist;
+    unsigned long long* const s_64 = sh.s64;
+    uint32_t* const s_ctl = sh.ctl;
 
     const uint32_t tx = tile % a.tiles_x, ty = tile / a.tiles_x;
     const uint32_t tid = threadIdx.x, lane = tid & 31u;
@@ -402,7 +556,8 @@ __device__ __forceinline__ void raster_tile(const RasterArgs& a, const uint32_t 
     if (MODE == 3) inside = !a.mask || !in_bounds;  // pixels outside the image weigh nothing
     if ((MODE == 2 || (MODE == 3 && a.mask)) && in_bounds) inside = (a.mask[px / 32 + py * a.mask_wpr] >> (px % 32)) & 1u;
     const uint32_t start = a.tile_start[tile], end = a.tile_start[tile + 1];
-    PixelState ps{1.0f, 0.0f, 0.0f, 0.0f, 0u, !in_bounds, 0u, 0u, 0u};
+    // A pixel takes entries while T >= 1/255; those outside the image start done.
+    PixelState ps{in_bounds ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f, 0u, 0u, 0u, 0u};
     if (ModeOf<MODE>::kWords) {
         for (uint32_t e = tid; e < kChunk; e += NT) {
             sm.acc0[0][e] = sm.acc0[1][e] = 0u;
@@ -416,7 +571,7 @@ __device__ __forceinline__ void raster_tile(const RasterArgs& a, const uint32_t 
 
     if (!LAZY || end - start <= a.lazy_min) {
         const uint32_t* ids = a.gaussian_ids + start;
-        composite_list<MODE, CULL, DETAIL, STATE, NT>(
+        composite_list<MODE, CULL, DETAIL, STATE || LAZY, NT>(
             a, sm, [&](uint32_t i) { return __ldg(ids + i); }, end - start, 0, fx, fy, wxf, wyf, inside, ps);
     } else if (end > start) {
         const uint2* pairs = a.pairs + start;
@@ -434,7 +589,7 @@ __device__ __forceinline__ void raster_tile(const RasterArgs& a, const uint32_t 
             for (uint32_t i = tid; i < n; i += NT) s_slab[i] = pair_value(pairs[i]);
             __syncthreads();
             bitonic_sort64<NT>(s_slab, n);
-            composite_list<MODE, CULL, DETAIL, STATE, NT>(a, sm, slab_id, n, 0, fx, fy, wxf, wyf, inside, ps);
+            composite_list<MODE, CULL, DETAIL, STATE || LAZY, NT>(a, sm, slab_id, n, 0, fx, fy, wxf, wyf, inside, ps);
         } else {
             unsigned long long cur = vmin;
             uint32_t pos = 0;
@@ -513,7 +668,7 @@ __device__ __forceinline__ void raster_tile(const RasterArgs& a, const uint32_t 
                 __syncthreads();
                 const uint32_t m = s_ctl[3];
                 bitonic_sort64<NT>(s_slab, m);
-                if (composite_list<MODE, CULL, DETAIL, STATE, NT>(a, sm, slab_id, m, pos, fx, fy, wxf, wyf,
+                if (composite_list<MODE, CULL, DETAIL, STATE || LAZY, NT>(a, sm, slab_id, m, pos, fx, fy, wxf, wyf,
                                                                   inside, ps))
                     break;
                 pos += m;
@@ -542,7 +697,7 @@ __device__ __forceinline__ void raster_tile(const RasterArgs& a, const uint32_t 
         // With one CTA per tile, 256 per entry the tile walks. The same
         // count for either list order.
         const uint32_t n_list = end - start;
-        uint32_t e = ps.done ? ps.last : n_list;
+        uint32_t e = ps.T < 1.0f / 255.0f ? ps.last : n_list;
         e = __reduce_max_sync(0xffffffffu, e);
         __syncthreads();
         if (tid == 0) s_ctl[0] = 0;
@@ -597,24 +752,31 @@ __global__ __launch_bounds__(NT) void raster_kernel(RasterArgs a) {
     raster_tile<MODE, CULL, DETAIL, STATE, LAZY, NT>(a, tile, sub);
 }
 
+template <int MODE, bool CULL, bool DETAIL, bool STATE, bool LAZY, uint32_t NT>
+cudaError_t raster_go(const RasterArgs& a, uint32_t tiles, cudaStream_t st) {
+    constexpr size_t smem = sizeof(TileShared<MODE, CULL, LAZY, NT>);
+    auto kernel = raster_kernel<MODE, CULL, DETAIL, STATE, LAZY, NT>;
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    kernel<<<tiles * (256 / NT), NT, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
 template <int MODE, bool LAZY>
-void raster_dispatch(const RasterArgs& a, uint32_t tiles, cudaStream_t st) {
+cudaError_t raster_dispatch(const RasterArgs& a, uint32_t tiles, cudaStream_t st) {
     // The per-pixel state (for the adjoint, and in mode 3 for read-backs of
     // the frame) and the pair diagnostics are kept by one CTA per tile.
     constexpr bool kState = MODE == 0 || MODE == 3;
-    const bool state = kState && (a.final_t || a.n_contrib);
     if (a.detail) {
-        if (a.cull) raster_kernel<MODE, true, true, kState, LAZY, 256><<<tiles, 256, 0, st>>>(a);
-        else raster_kernel<MODE, false, true, kState, LAZY, 256><<<tiles, 256, 0, st>>>(a);
-    } else if (state) {
-        raster_kernel<MODE, true, false, kState, LAZY, 256><<<tiles, 256, 0, st>>>(a);
-    } else if (a.split == 4) {
-        raster_kernel<MODE, true, false, false, LAZY, 64><<<tiles * 4, 64, 0, st>>>(a);
-    } else if (a.split == 2) {
-        raster_kernel<MODE, true, false, false, LAZY, 128><<<tiles * 2, 128, 0, st>>>(a);
-    } else {
-        raster_kernel<MODE, true, false, false, LAZY, 256><<<tiles, 256, 0, st>>>(a);
+        return a.cull ? raster_go<MODE, true, true, kState, LAZY, 256>(a, tiles, st)
+                      : raster_go<MODE, false, true, kState, LAZY, 256>(a, tiles, st);
     }
+    if (kState && (a.final_t || a.n_contrib)) return raster_go<MODE, true, false, kState, LAZY, 256>(a, tiles, st);
+    if (a.split == 4) return raster_go<MODE, true, false, false, LAZY, 64>(a, tiles, st);
+    if (a.split == 2) return raster_go<MODE, true, false, false, LAZY, 128>(a, tiles, st);
+    return raster_go<MODE, true, false, false, LAZY, 256>(a, tiles, st);
 }
 
 }  // namespace
@@ -627,18 +789,18 @@ cudaError_t launch_raster(int mode, const RasterArgs& args, cudaStream_t stream)
     if (a.split != 1 && a.split != 2 && a.split != 4) return cudaErrorInvalidValue;
     if (!a.ext) return cudaErrorInvalidValue;
     const bool lazy = a.pairs != nullptr;
+    cudaError_t e = cudaErrorInvalidValue;
     switch (mode) {
-        case 0: lazy ? raster_dispatch<0, true>(a, tiles, stream) : raster_dispatch<0, false>(a, tiles, stream); break;
-        case 1: lazy ? raster_dispatch<1, true>(a, tiles, stream) : raster_dispatch<1, false>(a, tiles, stream); break;
-        case 2: lazy ? raster_dispatch<2, true>(a, tiles, stream) : raster_dispatch<2, false>(a, tiles, stream); break;
+        case 0: e = lazy ? raster_dispatch<0, true>(a, tiles, stream) : raster_dispatch<0, false>(a, tiles, stream); break;
+        case 1: e = lazy ? raster_dispatch<1, true>(a, tiles, stream) : raster_dispatch<1, false>(a, tiles, stream); break;
+        case 2: e = lazy ? raster_dispatch<2, true>(a, tiles, stream) : raster_dispatch<2, false>(a, tiles, stream); break;
         case 3:
-            if (!a.afg || !a.abg || lazy) return cudaErrorInvalidValue;
-            raster_dispatch<3, false>(a, tiles, stream);
+            if (a.afg && a.abg && !lazy) e = raster_dispatch<3, false>(a, tiles, stream);
             break;
-        default: return cudaErrorInvalidValue;
+        default: break;
     }
-    note_launches(1);
-    return cudaGetLastError();
+    if (e == cudaSuccess) note_launches(1);
+    return e;
 }
 
 }  // namespace sfk
