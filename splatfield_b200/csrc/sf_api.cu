@@ -163,11 +163,9 @@ struct sf_scratch_t {
         size_t stage_words = 0;
         sf_view* views = nullptr;     // pinned, one per frame of the batch
         uint32_t* frame_words = nullptr;  // pinned, 16 per frame of the batch
-        // Device ring the graph's last node saves each frame's words to
-        // (slot = *ring_counter, which it then increments), read back once a
-        // run of frames has finished.
+        // Device ring each frame of a path saves its words to, read back once
+        // a run of frames has finished.
         uint32_t* ring = nullptr;
-        uint32_t* ring_counter = nullptr;
         uint32_t batch_cap = 0;
     } fg;
     uint32_t* bitmap = nullptr;
@@ -217,6 +215,8 @@ struct sf_scan_t {
 // ---------------------------------------------------------------- helpers
 
 namespace {
+
+constexpr uint32_t kStatusWords = 24;  // a scratch's 16 status words and four 64-bit pair statistics
 
 cudaError_t ensure_lut(sf_ctx ctx) {
     if (ctx->lut) return cudaSuccess;
@@ -325,8 +325,9 @@ cudaError_t scratch_build(sf_scratch s, uint32_t total, uint32_t w, uint32_t h) 
     const uint32_t scan_n = (uint32_t)std::max<size_t>(total, tiles + 1);
     if ((e = cudaMalloc(&s->scan_tmp, scan_temp_bytes(scan_n))) != cudaSuccess) return e;
     if (!s->words) {
-        if ((e = dalloc(&s->stats, 4)) != cudaSuccess) return e;
-        if ((e = dalloc(&s->words, 16)) != cudaSuccess) return e;
+        // One block, cleared together at the start of a frame graph.
+        if ((e = dalloc(&s->words, kStatusWords)) != cudaSuccess) return e;
+        s->stats = reinterpret_cast<unsigned long long*>(s->words + 16);
         if ((e = cudaMallocHost(reinterpret_cast<void**>(&s->host_words), 64)) != cudaSuccess) return e;
     }
     // Capacity: keep the larger of the growth hint and the reference's first
@@ -346,8 +347,8 @@ int prepare_binned(sf_scratch s, uint32_t n, uint32_t tiles, cudaStream_t st, bo
     unsigned long long* total_dev = reinterpret_cast<unsigned long long*>(words + 4);
     SF_CK(launch_bin_count(s->bbox, n, s->tiles_x, tiles, s->bin_chunks, s->bin_hist, st));
     SF_CK(launch_bin_colscan(s->bin_hist, s->bin_chunks, tiles, s->bin_cnt, s->bin_lists, words, st));
-    SF_CK(exclusive_scan(nullptr, s->bin_cnt, s->tile_start, tiles + 1, nullptr, tiles + 1, s->scan_tmp,
-                         total_dev, words + 1, st));
+    // The capacity follows the total below: the starts are not cut.
+    SF_CK(launch_tile_scan(s->bin_cnt, tiles + 1, 0xffffffffu, s->tile_start, total_dev, st));
     SF_CK(cudaMemcpyAsync(s->host_words, words, 64, cudaMemcpyDeviceToHost, st));
     SF_CK(cudaStreamSynchronize(st));
     const uint32_t* hw = s->host_words;
@@ -376,9 +377,12 @@ int prepare_binned(sf_scratch s, uint32_t n, uint32_t tiles, cudaStream_t st, bo
         if (order == SF_ORDER_HYBRID) grids[kSortClasses - 1] = 0;
         // The longest list is known here: the segmented sort runs only when
         // some list is long enough to gain from it.
+        GiantState giant = s->giant;
+        giant.min_list = kGiantMinAlone;
+        if (!s->sort_streams.s[0]) SF_CK(sort_streams_create(&s->sort_streams));
         SF_CK(launch_tile_sorts(grids, s->bin_lists, words, tiles, s->tile_start, (uint32_t)s->cap, pairs,
                                 s->gid_e, want_tile_ids ? s->tid_e : nullptr, s->tid_e, s->ctx->sm_count, st,
-                                nullptr, hw[6] > kGiantMinList ? &s->giant : nullptr));
+                                &s->sort_streams, hw[6] > kGiantMinAlone ? &giant : nullptr));
         s->tids = want_tile_ids ? s->tid_e : nullptr;
         s->gids = s->gid_e;
     }
@@ -544,10 +548,9 @@ int accumulate(sf_scratch s, const sf_isects* is, uint32_t w, uint32_t h, sf_acc
 //
 // A binned RGB frame with no host step in the middle: projection, counts,
 // scans, placement against the current capacity (device-side guard, tile
-// starts clamped), per-tile sorts as persistent kernels reading their class
-// sizes on the device (the classes on side streams), raster, and the status
-// words saved to a device ring — captured once and replayed with one launch
-// per frame on the caller's stream. The host reads the words after the frame
+// starts cut there), per-tile sorts as persistent kernels reading their class
+// sizes on the device (the classes on side streams) and raster — captured once
+// and replayed with one launch per frame on the caller's stream. The host reads the words after the frame
 // (or after a run of frames); a frame that outgrew the capacity grows it and
 // runs again (the graph is captured anew).
 
@@ -571,7 +574,6 @@ int frame_graph_capture(sf_splats sp, sf_scratch s) {
     if (!g.stream) SF_CK(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
     if (!g.view_dev) SF_CK(dalloc(&g.view_dev, 1));
     if (!g.ring) SF_CK(dalloc(&g.ring, 16 * (size_t)kFrameRing));
-    if (!g.ring_counter) SF_CK(dalloc(&g.ring_counter, 1));
     if (!g.view_host) SF_CK(cudaMallocHost(reinterpret_cast<void**>(&g.view_host), sizeof(sf_view)));
     if (!s->sort_streams.s[0]) SF_CK(sort_streams_create(&s->sort_streams));
     const uint32_t n = sp->n;
@@ -586,8 +588,7 @@ int frame_graph_capture(sf_splats sp, sf_scratch s) {
     // pinned slot of the caller's choosing), outside the graph.
     const uint64_t launches0 = launches();
     SF_CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = cudaMemsetAsync(words, 0, 64, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(s->stats, 0, 32, st);
+    cudaError_t e = cudaMemsetAsync(words, 0, 4 * kStatusWords, st);
     ProjOut po{s->depth_keys, s->tile_counts, s->bbox, s->geo0, s->geo1, s->color, words, s->ext};
     sf_view dummy{};
     if (e == cudaSuccess) e = launch_project(dummy, sp->attr, sp->geom, sp->sh, n, sp->K, po, st, g.view_dev);
@@ -595,17 +596,14 @@ int frame_graph_capture(sf_splats sp, sf_scratch s) {
     if (e == cudaSuccess)
         e = launch_bin_colscan(s->bin_hist, s->bin_chunks, tiles, s->bin_cnt, s->bin_lists, words, st);
     if (e == cudaSuccess)
-        e = exclusive_scan(nullptr, s->bin_cnt, s->tile_start, tiles + 1, nullptr, tiles + 1, s->scan_tmp, total,
-                           words + 1, st);
-    if (e == cudaSuccess) e = launch_clamp_count(total, cap, words + 2, words + 1, st);
+        e = launch_tile_scan(s->bin_cnt, tiles + 1, cap, s->tile_start, total, st);
     uint2* pairs = reinterpret_cast<uint2*>(s->tid_a);
     if (e == cudaSuccess)
         e = launch_bin_place(s->bbox, s->depth_keys, n, s->tiles_x, tiles, s->bin_chunks, s->bin_hist,
                              s->tile_start, cap, pairs, words + 1, st);
-    if (e == cudaSuccess) e = launch_clamp_starts(s->tile_start, tiles + 1, cap, st);
     if (e == cudaSuccess && order != SF_ORDER_IN_RASTER) {
         uint32_t grids[kSortClasses];
-        for (int k = 0; k < kSortClasses; ++k) grids[k] = tiles;
+        tile_sort_bounds(n, tiles, grids);
         if (order == SF_ORDER_HYBRID) grids[kSortClasses - 1] = 0;
         e = launch_tile_sorts(grids, s->bin_lists, words, tiles, s->tile_start, cap, pairs, s->gid_e, nullptr,
                               s->tid_e, s->ctx->sm_count, st, &s->sort_streams, giant ? &s->giant : nullptr);
@@ -634,7 +632,6 @@ int frame_graph_capture(sf_splats sp, sf_scratch s) {
         }
         e = launch_raster(0, a, st);
     }
-    if (e == cudaSuccess) e = launch_save_words(words, g.ring, g.ring_counter, kFrameRing, st);
     cudaGraph_t graph = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(st, &graph);
     g.kernels = (uint32_t)(launches() - launches0);
@@ -845,6 +842,7 @@ int frames_graph_render(sf_splats sp, sf_scratch s, const sf_camera* cams, uint3
         SF_CK(cudaEventRecord(s->fork, st));
         SF_CK(cudaStreamWaitEvent(streams[1], s->fork, 0));
     }
+    uint32_t slots[2] = {0, 0};  // frames of this run saved to each pipe's ring
     for (uint32_t i = 0; i < count; ++i) {
         const int slot = (int)(i & 1u);
         const int p = pipe_of(i);
@@ -859,12 +857,12 @@ int frames_graph_render(sf_splats sp, sf_scratch s, const sf_camera* cams, uint3
                 SF_CK(cudaStreamSynchronize(streams[1]));
                 SF_CK(read_rings(pipes, pipe_of, i - kFrameRing, i, g.frame_words));
             }
-            SF_CK(cudaMemsetAsync(pipes[0]->fg.ring_counter, 0, 4, streams[0]));
-            if (two) SF_CK(cudaMemsetAsync(pipes[1]->fg.ring_counter, 0, 4, streams[1]));
+            slots[0] = slots[1] = 0;
         }
         SF_CK(cudaMemcpyAsync(P->fg.view_dev, g.views + i, sizeof(sf_view), cudaMemcpyHostToDevice, ps));
         SF_CK(cudaGraphLaunch(P->fg.exec, ps));
         note_launches(P->fg.kernels);
+        SF_CK(cudaMemcpyAsync(P->fg.ring + 16 * (size_t)slots[p]++, P->words, 64, cudaMemcpyDeviceToDevice, ps));
         if (!host_out) continue;
         // Frames i and i + 2 share a staging image (and, with two pipes, a
         // pipe).
@@ -1131,8 +1129,7 @@ int sf_scratch_destroy(sf_scratch s) {
     sf_scratch_destroy(s->twin);
     scratch_free_frame(s);
     scratch_free_isects(s);
-    dfree(s->words);
-    dfree(s->stats);
+    dfree(s->words);  // and the stats behind them
     if (s->host_words) cudaFreeHost(s->host_words);
     sort_streams_destroy(&s->sort_streams);
     if (s->fg.exec) cudaGraphExecDestroy(s->fg.exec);
@@ -1151,7 +1148,6 @@ int sf_scratch_destroy(sf_scratch s) {
     if (s->fg.views) cudaFreeHost(s->fg.views);
     if (s->fg.frame_words) cudaFreeHost(s->fg.frame_words);
     dfree(s->fg.ring);
-    dfree(s->fg.ring_counter);
     delete s;
     return SF_OK;
 }

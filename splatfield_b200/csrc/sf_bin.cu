@@ -12,7 +12,8 @@
 //      shared-memory histogram, written as hist[c][tile].
 //   2. bin_colscan: per tile, the exclusive prefix of hist over the chunks (in
 //      place) and the tile's total; tiles are filed into size classes.
-//      An exclusive scan of the totals (sfk::exclusive_scan) gives tile_start.
+//      An exclusive scan of the totals (tile_scan) gives tile_start, cut at
+//      the capacity.
 //   3. bin_place: chunk c re-walks its pairs and drops each (depth key, splat
 //      id) at tile_start[t] + hist[c][t] + a shared-memory cursor. The order
 //      inside a tile is not yet fixed.
@@ -813,7 +814,7 @@ static_assert(kSortClasses == 7, "class table");
 // ---- segmented sort of the longest lists
 //
 // One CTA sorting a list of 10^5 entries takes milliseconds. Lists of the
-// longest class past kGiantMinList entries (the first GiantState::lists of
+// longest class past GiantState::min_list entries (the first GiantState::lists of
 // them) are instead sorted over all SMs:
 //   0. giant_select (one CTA): picks those lists, gives each its first chunk
 //      of kGiantChunk entries in one numbering over the picked lists, resets
@@ -837,7 +838,8 @@ static_assert(kSortClasses == 7, "class table");
 constexpr uint32_t kGiantThreads = 256, kGiantItems = 8, kGiantChunk = kGiantThreads * kGiantItems;
 constexpr uint32_t kGiantPlanThreads = 1024;
 static_assert(kGiantBins == 2 * kGiantPlanThreads, "two buckets per plan thread");
-static_assert(kGiantMinList >= kClass2, "the segmented lists belong to the longest class");
+static_assert(kGiantMinList >= kClass2 && kGiantMinAlone >= kClass2,
+              "the segmented lists belong to the longest class");
 
 __device__ __forceinline__ uint32_t giant_shift(uint32_t mn, uint32_t mx) {
     const uint32_t range = mx - mn;
@@ -892,7 +894,7 @@ __global__ __launch_bounds__(1024) void giant_select_kernel(const uint32_t* __re
             start = tile_start[t];
             const uint32_t end = tile_start[t + 1];
             n = end - start;
-            big = end <= capacity && end >= start && n > kGiantMinList;
+            big = end <= capacity && end >= start && n > gs.min_list;
         }
         uint32_t nbig;
         const uint32_t r = picked + block_scan<1024>(big ? 1u : 0u, s32, nbig);
@@ -1161,9 +1163,14 @@ cudaError_t smem_opt_in(const void* fn, size_t smem) {
 
 }  // namespace
 
+// Two chunks per SM, of at least kMinBinChunk splats: a block's 32 warps take
+// 32 splats each at a time, so smaller chunks leave most of its warps idle and
+// give the column scan more rows to add (3001 splats: 94 chunks -> 6, count,
+// column scan and place 14.4 -> 13.6 us).
+constexpr uint32_t kMinBinChunk = 512;
 uint32_t bin_chunks(uint32_t n, int sm_count) {
     const uint32_t c = (uint32_t)std::max(1, 2 * sm_count);
-    return std::max(1u, std::min(c, (n + 31) / 32));
+    return std::max(1u, std::min(c, (n + kMinBinChunk - 1) / kMinBinChunk));
 }
 
 uint32_t bin_chunk_size(uint32_t n, uint32_t chunks) { return ((n + chunks - 1) / chunks + 31) / 32 * 32; }
@@ -1181,6 +1188,10 @@ uint32_t giant_seg_cap(uint32_t lists) { return (1u << 30) / kGiantSegTarget + l
 uint32_t bin_class_limit(int k) {
     const uint32_t lim[kSortClasses - 1] = {kClassWarp, kClassS, kClass0, kClassM, kClass1, kClass2};
     return k >= 0 && k < kSortClasses - 1 ? lim[k] : 0xffffffffu;
+}
+
+void tile_sort_bounds(uint32_t n, uint32_t tiles, uint32_t grids[kSortClasses]) {
+    for (int k = 0; k < kSortClasses; ++k) grids[k] = k == 0 || n > bin_class_limit(k - 1) ? tiles : 0u;
 }
 
 cudaError_t launch_bin_count(const uint2* bbox, uint32_t n, uint32_t tiles_x, uint32_t tiles, uint32_t chunks,
@@ -1225,19 +1236,63 @@ __global__ void clamp_count_kernel(const unsigned long long* total, uint32_t cap
     *n32 = (uint32_t)(t < cap ? t : cap);
 }
 
-__global__ void save_words_kernel(const uint32_t* __restrict__ words, uint32_t* __restrict__ ring,
-                                  uint32_t* counter, uint32_t ring_frames) {
-    const uint32_t idx = *counter;
-    if (idx < ring_frames)
-        for (uint32_t k = 0; k < 16; ++k) ring[(size_t)idx * 16 + k] = words[k];
-    *counter = idx + 1;
-}
-
-__global__ void clamp_starts_kernel(uint32_t* tile_start, uint32_t count, uint32_t cap) {
+// Tile starts: start[i] = min(sum of cnt[0, i), cap) for i < n (cnt[n - 1] is
+// the closing zero), *total the 64-bit sum. One CTA, 4096 counts per step: a
+// frame has at most 49152 tiles, and without partitions there is no look-back
+// state to clear before it and no separate pass to cut the starts (a memset,
+// the scan and the cut took 8 us of a frame's chain, this kernel 3 us at
+// 1080p). Starts at the capacity make the placement drop every later pair and
+// the sorts and the raster stay within it.
+constexpr uint32_t kTileScanThreads = 1024;
+__global__ __launch_bounds__(kTileScanThreads) void tile_scan_kernel(const uint32_t* __restrict__ cnt, uint32_t n,
+                                                                     uint32_t cap, uint32_t* __restrict__ start,
+                                                                     unsigned long long* total) {
     pdl_trigger();
     pdl_wait();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < count && tile_start[i] > cap) tile_start[i] = cap;
+    __shared__ unsigned long long s_warp[32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    unsigned long long carry = 0;
+    for (uint32_t i0 = 0; i0 < n; i0 += 4 * kTileScanThreads) {
+        const uint32_t i = i0 + 4 * tid;
+        uint32_t c[4] = {0u, 0u, 0u, 0u};
+        if (i + 4 <= n) {
+            const uint4 q = *reinterpret_cast<const uint4*>(cnt + i);
+            c[0] = q.x;
+            c[1] = q.y;
+            c[2] = q.z;
+            c[3] = q.w;
+        } else {
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k)
+                if (i + k < n) c[k] = cnt[i + k];
+        }
+        const unsigned long long own = ((unsigned long long)c[0] + c[1]) + ((unsigned long long)c[2] + c[3]);
+        unsigned long long incl = own;
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const unsigned long long v = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += v;
+        }
+        __syncthreads();  // the last step's totals have been read
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        unsigned long long w = s_warp[lane];
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const unsigned long long v = __shfl_up_sync(0xffffffffu, w, d);
+            if (lane >= d) w += v;
+        }
+        unsigned long long run = carry + (incl - own);
+        const unsigned long long before = __shfl_sync(0xffffffffu, w, (warp + 31u) & 31u);
+        if (warp > 0) run += before;
+        carry += __shfl_sync(0xffffffffu, w, 31);
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            if (i + k < n) start[i + k] = run < cap ? (uint32_t)run : cap;
+            run += c[k];
+        }
+    }
+    if (tid == 0) *total = carry;
 }
 
 }  // namespace
@@ -1249,15 +1304,9 @@ cudaError_t launch_clamp_count(const unsigned long long* total, uint32_t cap, ui
     return e;
 }
 
-cudaError_t launch_save_words(const uint32_t* words, uint32_t* ring, uint32_t* counter, uint32_t ring_frames,
-                              cudaStream_t st) {
-    save_words_kernel<<<1, 1, 0, st>>>(words, ring, counter, ring_frames);
-    note_launches(1);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_clamp_starts(uint32_t* tile_start, uint32_t count, uint32_t cap, cudaStream_t st) {
-    const cudaError_t e = launch_pdl(clamp_starts_kernel, (count + 255) / 256, 256, 0, st, tile_start, count, cap);
+cudaError_t launch_tile_scan(const uint32_t* cnt, uint32_t n, uint32_t cap, uint32_t* start,
+                             unsigned long long* total, cudaStream_t st) {
+    const cudaError_t e = launch_pdl(tile_scan_kernel, 1, kTileScanThreads, 0, st, cnt, n, cap, start, total);
     note_launches(1);
     return e;
 }
@@ -1293,7 +1342,7 @@ cudaError_t smem_attr(K kernel, size_t smem) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
-// The longest class: the segmented sort for its lists past kGiantMinList
+// The longest class: the segmented sort for its lists past gs->min_list
 // entries (the first gs->lists of them), the one-CTA global form for the
 // rest. grid: the class's tile count (or an upper bound); 0 leaves the class
 // unsorted.
@@ -1324,6 +1373,8 @@ cudaError_t launch_giant_sorts(uint32_t grid, const uint32_t* list, const uint32
         note_launches(7);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
+    // Every list of the class is past min_list and taken.
+    if (seg && gs->min_list <= kClass2 && grid <= gs->lists) return cudaSuccess;
     global_form<<<std::min(grid, sms), kThreadsGiant, kGiantSmem, st>>>(list, n, tile_start, capacity, pairs, ids,
                                                                          tids_out, keys_tmp,
                                                                          seg ? gs->taken : nullptr);
@@ -1341,10 +1392,11 @@ cudaError_t launch_tile_sorts(const uint32_t grids[kSortClasses], const uint32_t
     // Each form reads and overwrites only its own tiles' ranges, so the
     // classes may run concurrently.
     cudaStream_t s1 = st, s2 = st, s3 = st, s4 = st;
+    const bool used[4] = {grids[4] > 0, grids[5] > 0 || grids[0] > 0, grids[6] > 0 || grids[1] > 0, grids[3] > 0};
     if (side && side->s[0]) {
         if ((e = cudaEventRecord(side->e[0], st)) != cudaSuccess) return e;
         for (int k = 0; k < 4; ++k)
-            if ((e = cudaStreamWaitEvent(side->s[k], side->e[0], 0)) != cudaSuccess) return e;
+            if (used[k] && (e = cudaStreamWaitEvent(side->s[k], side->e[0], 0)) != cudaSuccess) return e;
         s1 = side->s[0];
         s2 = side->s[1];
         s3 = side->s[2];
@@ -1380,6 +1432,7 @@ cudaError_t launch_tile_sorts(const uint32_t grids[kSortClasses], const uint32_t
     if (e != cudaSuccess) return e;
     if (side && side->s[0]) {
         for (int k = 0; k < 4; ++k) {
+            if (!used[k]) continue;
             if ((e = cudaEventRecord(side->e[1 + k], side->s[k])) != cudaSuccess) return e;
             if ((e = cudaStreamWaitEvent(st, side->e[1 + k], 0)) != cudaSuccess) return e;
         }

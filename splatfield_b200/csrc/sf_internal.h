@@ -205,13 +205,19 @@ constexpr uint32_t kBinSharedMax = 12288;
 // (all zero on entry).
 cudaError_t launch_bin_count(const uint2* bbox, uint32_t n, uint32_t tiles_x, uint32_t tiles, uint32_t chunks,
                              uint32_t* hist, cudaStream_t st);
-// Segmented sort of the longest lists (sf_bin.cu): each list past 24576
+// Segmented sort of the longest lists (sf_bin.cu): each list past min_list
 // entries (up to `lists` of them per frame) gets a key histogram of
 // kGiantBins buckets, cut into segments of about kGiantSegTarget entries that
 // are sorted on separate CTAs; shorter lists of the longest class, and any
 // past `lists`, are sorted by one CTA each.
 constexpr uint32_t kGiantBins = 2048, kGiantSegTarget = 4096, kGiantMaxLists = 4096;
 constexpr uint32_t kGiantMinList = 24576;
+// Outside a graph (sf_prepare_isects and the calls built on it) the longest
+// list is known before the sorts and nothing else hides it: a list of 24576
+// entries takes one CTA 93 us and the segmented chain 60 us (label-sized frame
+// of 1M splats, 15 such lists), so every list of the longest class goes to the
+// chain.
+constexpr uint32_t kGiantMinAlone = 12288;
 struct GiantState {
     uint32_t* ctrl = nullptr;  // [4]: lists taken, chunks, short segments, long segments
     uint4* sel = nullptr;      // [lists]: (tile, first slot, entries, first chunk)
@@ -221,6 +227,7 @@ struct GiantState {
     uint4* segs = nullptr;     // [seg_cap]: (tile, first slot, entries, 0)
     uint32_t lists = 0;
     uint32_t seg_cap = 0;
+    uint32_t min_list = kGiantMinList;  // lists longer than this are segmented
 };
 // Whether a captured graph includes the segmented sort, from the longest
 // list of the frames seen so far (`on`: the last graph had it): on past
@@ -243,26 +250,21 @@ cudaError_t launch_bin_colscan(uint32_t* hist, uint32_t chunks, uint32_t tiles, 
 cudaError_t launch_bin_place(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
                              uint32_t tiles, uint32_t chunks, const uint32_t* hist, const uint32_t* tile_start,
                              uint32_t capacity, uint2* pairs, uint32_t* err, cudaStream_t st);
-// grids[k]: CTAs launched for class k (the class count when the host knows
-// it, else `tiles`; CTAs past the device count exit); grids[3] = 0 leaves
-// the longest lists unsorted.
-// Device-side capacity handling when the intersection total is not read
-// on the host first: n32 = min(total, cap) with SF_DEV_ERR_CAPACITY set past
-// it, and tile starts cut back to the capacity (every slot below it holds a
-// placed pair, so the sorts and the raster stay inside the buffers).
+// Device-side capacity handling of the depth-sorted build when the
+// intersection total is not read on the host first: n32 = min(total, cap) with
+// SF_DEV_ERR_CAPACITY set past it.
 cudaError_t launch_clamp_count(const unsigned long long* total, uint32_t cap, uint32_t* n32, uint32_t* err,
                                cudaStream_t st);
-// A frame's 16 status words to slot *counter of a device ring (when it is
-// below ring_frames), then ++*counter: the last node of the frame graph, so
-// frames enqueued back to back keep their words on the device.
-cudaError_t launch_save_words(const uint32_t* words, uint32_t* ring, uint32_t* counter, uint32_t ring_frames,
-                              cudaStream_t st);
-cudaError_t launch_clamp_starts(uint32_t* tile_start, uint32_t count, uint32_t cap, cudaStream_t st);
+// Tile starts of a binned build: start[i] = min(sum of cnt[0, i), cap) for
+// i < n (n = tiles + 1, cnt[tiles] = 0), *total the 64-bit intersection count.
+// With starts cut at the capacity, every slot below it holds a placed pair, so
+// the sorts and the raster stay inside the buffers.
+cudaError_t launch_tile_scan(const uint32_t* cnt, uint32_t n, uint32_t cap, uint32_t* start,
+                             unsigned long long* total, cudaStream_t st);
 
-// Side streams the per-tile sort classes run on concurrently inside a
-// captured graph (the tail of one class overlaps the others); null runs them
-// in turn on one stream (outside a graph the extra event calls cost more
-// host time than the overlap gains).
+// Side streams the per-tile sort classes run on concurrently (the tail of one
+// class overlaps the others); streams whose classes are empty (grids of 0) are
+// not forked.
 struct SortStreams {
     cudaStream_t s[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaEvent_t e[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -270,6 +272,9 @@ struct SortStreams {
 cudaError_t sort_streams_create(SortStreams* ss);
 void sort_streams_destroy(SortStreams* ss);
 
+// Grid bounds of the size classes when their tile counts stay on the device:
+// every tile, or 0 for a class whose lists would be longer than n splats.
+void tile_sort_bounds(uint32_t n, uint32_t tiles, uint32_t grids[kSortClasses]);
 // pairs: the placed (depth key, splat id) per slot (overwritten for the
 // longest lists); ids / tids_out receive the sorted splat ids / tile ids
 // (tids_out may be null); keys_tmp: capacity u32 of scratch (may alias

@@ -347,21 +347,17 @@ cudaError_t enqueue_view(sf_round_t* r, RoundLane& L, uint32_t v, const sf_splat
         // the bound of each class and read the class sizes on the device.
         if ((e = launch_bin_count(L.bbox, n, tx, tiles, r->chunks, L.hist, st)) != cudaSuccess) return e;
         if ((e = launch_bin_colscan(L.hist, r->chunks, tiles, L.cnt, L.lists, words, st)) != cudaSuccess) return e;
-        if ((e = exclusive_scan(nullptr, L.cnt, L.tile_start, tiles + 1, nullptr, tiles + 1, L.scan_tmp, total,
-                                words + 1, st)) != cudaSuccess)
-            return e;
-        if ((e = launch_clamp_count(total, (uint32_t)L.cap, words + 2, words + 1, st)) != cudaSuccess) return e;
+        if ((e = launch_tile_scan(L.cnt, tiles + 1, (uint32_t)L.cap, L.tile_start, total, st)) != cudaSuccess) return e;
         uint2* pairs = reinterpret_cast<uint2*>(L.tid_a);
         if ((e = launch_bin_place(L.bbox, L.keys, n, tx, tiles, r->chunks, L.hist, L.tile_start, (uint32_t)L.cap,
                                   pairs, words + 1, st)) != cudaSuccess)
             return e;
-        if ((e = launch_clamp_starts(L.tile_start, tiles + 1, (uint32_t)L.cap, st)) != cudaSuccess) return e;
         // The adjoint's lists are sorted whatever the tuning's order.
         const uint32_t order = r->adjoint ? SF_ORDER_SORTED : r->tuning.raster_order;
         if (order != SF_ORDER_SORTED) lazy_pairs = pairs;
         if (order != SF_ORDER_IN_RASTER) {
             uint32_t grids[kSortClasses];
-            for (int k = 0; k < kSortClasses; ++k) grids[k] = tiles;
+            tile_sort_bounds(n, tiles, grids);
             if (order == SF_ORDER_HYBRID) grids[kSortClasses - 1] = 0;
             if ((e = launch_tile_sorts(grids, L.lists, words, tiles, L.tile_start, (uint32_t)L.cap, pairs, L.gid_e,
                                        nullptr, L.tid_e, r->sm_count, st, &L.sort_streams,
