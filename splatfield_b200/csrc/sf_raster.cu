@@ -13,9 +13,9 @@
 // into shared memory with cp.async (16-byte global -> shared copies that
 // need no registers), double-buffered: chunk c + 1 is in flight while chunk c
 // is composited, and the ids of chunk c + 2 are loaded a chunk ahead, so the
-// gather latency overlaps the walk instead of stalling every warp between two
-// barriers. Two barriers per chunk: one before reusing a buffer, one (with the
-// saturation count) before compositing it.
+// gather latency overlaps the walk. One barrier per chunk, with the saturation
+// count: past it chunk c is complete and chunk c - 1's buffer is free (mode 3
+// takes a second one, for its single-buffered sums).
 //
 // Per pair: the power of the splat's quadratic form at the pixel; a pair with
 // power above the splat's power_max (alpha < 1/255 for sure) is skipped;
@@ -432,20 +432,19 @@ __device__ bool composite_list(const RasterArgs& a, Stage<MODE, CULL, NT>& sm, I
     if (nchunks > 1) load_ids(1);
     for (uint32_t c = 0; c < nchunks; ++c) {
         const uint32_t b = c & 1u;
-        // The walk of chunk c - 1 is over: its buffer may be refilled and
-        // its sums are complete.
-        __syncthreads();
+        cp_async_wait<0>();  // this thread's copies of chunk c have landed
+        // One barrier: every thread's copies of chunk c are there, and the
+        // walk of chunk c - 1 is over, so its sums are complete and its buffer
+        // may be refilled.
+        const bool all_done = __syncthreads_count(done()) == NT;
         if ((kWords || kReal) && c > 0) flush(b ^ 1u, kChunk);
+        if (all_done) return true;
         if (c + 1 < nchunks) {
             issue(c + 1, b ^ 1u);
+            cp_async_commit();
             if (c + 2 < nchunks) load_ids(c + 2);
         }
-        cp_async_commit();
-        cp_async_wait<1>();  // this thread's copies of chunk c have landed
-        if (__syncthreads_count(done()) == NT) {
-            cp_async_wait<0>();
-            return true;
-        }
+        if (kReal) __syncthreads();  // the warps' sums of the last chunk have been read
         const uint32_t cnt = min(kChunk, count - c * kChunk);
         if (!EXACT && !done()) ps.last = c * kChunk + cnt;
         const uint32_t pos0 = list_off + c * kChunk + 1;
