@@ -1826,12 +1826,13 @@ int sf_localize(sf_splats s, sf_beta b, sf_stream stream, int* found, float cent
         if (s->n != b->n) return fail(SF_ERR_SHAPE, "splat count and posterior size differ");
         SF_CK(use_device(b->ctx->device));
         if (!b->loc_out) {
-            SF_CK(dalloc(&b->loc_partials, 4 * (size_t)b->blocks));
+            SF_CK(dalloc(&b->loc_partials, 4 * (size_t)localize_blocks(b->n, b->ctx->sm_count)));
             SF_CK(dalloc(&b->loc_out, 8));
             SF_CK(cudaMallocHost(reinterpret_cast<void**>(&b->loc_host), 8 * sizeof(double)));
         }
         cudaStream_t st = S(stream);
-        SF_CK(launch_localize(s->attr, b->a, b->b, b->n, b->loc_partials, b->blocks, b->loc_out, st));
+        SF_CK(launch_localize(s->attr, b->a, b->b, b->n, b->loc_partials, localize_blocks(b->n, b->ctx->sm_count),
+                              b->loc_out, st));
         SF_CK(cudaMemcpyAsync(b->loc_host, b->loc_out, 8 * sizeof(double), cudaMemcpyDeviceToHost, st));
         SF_CK(cudaStreamSynchronize(st));
         const double* o = b->loc_host;

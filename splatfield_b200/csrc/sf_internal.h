@@ -304,6 +304,7 @@ cudaError_t launch_eig(int mode, const float* a, const float* b, const uint32_t*
 cudaError_t launch_entropy(int mode, const float* a, const float* b, uint32_t n, const float* table, void* out,
                            cudaStream_t stream);
 uint32_t eig_blocks(uint32_t n, int sm_count);
+uint32_t localize_blocks(uint32_t n, int sm_count);
 // Posterior heatmap colours and foreground tint (src/seg/paint.rs).
 cudaError_t launch_paint_posterior(const float* a, const float* b, uint32_t n, float4* color,
                                    cudaStream_t stream);

@@ -68,10 +68,8 @@ using namespace sfm;
 //     0.5 ln(2 pi) terms of the three lgammas leave one constant.
 // psi keeps its recurrence (no division for x >= 6, most arguments).
 // Arguments past 2^32 take the per-term forms (the fractions' products of
-// eight factors stay below 2^260 under that bound). Measured on the
-// 20-view FP64 round: 3.68 -> 3.48 ms, with the EIG kernels held to five
-// blocks per SM (the fractions raise register use; at two blocks per SM
-// the round took 3.71 ms, at three 3.54, at four 3.52).
+// eight factors stay below 2^260 under that bound). Measured on a 20-view
+// FP64 round: 3.68 -> 3.48 ms.
 __device__ __forceinline__ double lgamma_terms(double x) {
     const double z = x - 1.0;
     double series = 0.9999999999998099;
@@ -159,76 +157,91 @@ __device__ __forceinline__ double block_sum(double v, double* s_warp) {
     return total;
 }
 
-// entropy_delta_kernel (beta.rs:152-201): per splat with eps > 0,
-// dH = max(0, H(a,b) - H(k a, k b)), k = 1 + eps/(a+b).
-template <int MODE>
-__global__ __launch_bounds__(kEigThreads, 5) void eig_kernel(const float* __restrict__ a,
-                                                          const float* __restrict__ b,
-                                                          const uint32_t* __restrict__ resp,
-                                                          const uint32_t* __restrict__ resp2,
-                                                          uint32_t n, float scale,
-                                                          const float* __restrict__ table,
-                                                          double* __restrict__ partials,
-                                                          const void* __restrict__ h0) {
-    __shared__ double s_warp[kEigThreads / 32];
-    double acc = 0.0;
-    const uint32_t stride = gridDim.x * kEigThreads;
-    for (uint32_t i = blockIdx.x * kEigThreads + threadIdx.x; i < n; i += stride) {
-        // eps words; with an evidence split, eps = fg + bg exactly.
-        const uint32_t bits = resp[i] + (resp2 ? resp2[i] : 0u);
-        if (bits == 0u) continue;
-        const float ai = a[i], bi = b[i];
-        if (MODE == SF_EIG_LUT_F32) {
-            const float eps = (float)bits / scale;
-            const float k = 1.0f + eps / (ai + bi);
-            const float hab = h0 ? static_cast<const float*>(h0)[i] : table_entropy_d(ai, bi, table);
-            const float d = max_(hab - table_entropy_d(ai * k, bi * k, table), 0.0f);
-            acc += (double)d;
-        } else {
-            const double eps = (double)bits / (double)scale;
-            const double ad = ai, bd = bi;
-            const double k = 1.0 + eps / (ad + bd);
-            const double hab = h0 ? static_cast<const double*>(h0)[i] : beta_entropy_d(ad, bd);
-            const double d = hab - beta_entropy_d(ad * k, bd * k);
-            acc += d > 0.0 ? d : 0.0;
-        }
+// Responsibilities of splat i: fixed-point words (fg + bg exactly, bg may be
+// null), or the real-valued ones of the adjoint (eps = fg + bg with no scale).
+struct EpsWords {
+    const uint32_t *fg, *bg;
+    float scale;
+    __device__ __forceinline__ uint32_t bits(uint32_t i) const { return fg[i] + (bg ? bg[i] : 0u); }
+    __device__ __forceinline__ bool any(uint32_t i) const { return bits(i) != 0u; }
+    __device__ __forceinline__ float f32(uint32_t i) const { return (float)bits(i) / scale; }
+    __device__ __forceinline__ double f64(uint32_t i) const { return (double)bits(i) / (double)scale; }
+};
+struct EpsReal {
+    const float *fg, *bg;
+    __device__ __forceinline__ bool any(uint32_t i) const { return fg[i] + (bg ? bg[i] : 0.0f) > 0.0f; }
+    __device__ __forceinline__ float f32(uint32_t i) const { return fg[i] + (bg ? bg[i] : 0.0f); }
+    __device__ __forceinline__ double f64(uint32_t i) const { return (double)fg[i] + (bg ? (double)bg[i] : 0.0); }
+};
+
+// dH = max(0, H(a,b) - H(k a, k b)), k = 1 + eps/(a+b), of splat i.
+template <int MODE, typename Eps>
+__device__ __forceinline__ double entropy_delta(uint32_t i, const Eps& eps, const float* __restrict__ a,
+                                                const float* __restrict__ b, const float* __restrict__ table,
+                                                const void* __restrict__ h0) {
+    const float ai = a[i], bi = b[i];
+    if (MODE == SF_EIG_LUT_F32) {
+        const float k = 1.0f + eps.f32(i) / (ai + bi);
+        const float hab = h0 ? static_cast<const float*>(h0)[i] : table_entropy_d(ai, bi, table);
+        return (double)max_(hab - table_entropy_d(ai * k, bi * k, table), 0.0f);
     }
-    const double total = block_sum(acc, s_warp);
-    if (threadIdx.x == 0) partials[blockIdx.x] = total;
+    const double ad = ai, bd = bi;
+    const double k = 1.0 + eps.f64(i) / (ad + bd);
+    const double hab = h0 ? static_cast<const double*>(h0)[i] : beta_entropy_d(ad, bd);
+    const double d = hab - beta_entropy_d(ad * k, bd * k);
+    return d > 0.0 ? d : 0.0;
 }
 
-// entropy_delta_kernel over real-valued responsibilities (the adjoint of a
-// per-splat scalar feature, sf_backward.cu): eps = fg + bg directly, with no
-// fixed-point scale; the LUT form adds in f32, the FP64 form in f64.
-template <int MODE>
-__global__ __launch_bounds__(kEigThreads, 5) void eig_real_kernel(const float* __restrict__ a,
-                                                               const float* __restrict__ b,
-                                                               const float* __restrict__ fg,
-                                                               const float* __restrict__ bg, uint32_t n,
-                                                               const float* __restrict__ table,
-                                                               double* __restrict__ partials,
-                                                               const void* __restrict__ h0) {
+// entropy_delta_kernel (beta.rs:152-201): the sum of dH over the splats with
+// eps > 0. A view gives weight to few of them (7 to 33%), scattered among the
+// others, and the entropies are long (FP64: 4 logs and 6 divisions), so a
+// warp that evaluated its splats where they lie would run almost every 32 of
+// them for a few live lanes. Each warp instead queues the splats that have
+// weight, in index order, and evaluates 32 at a time. The partition and the
+// order of the sums depend on n alone, so a view's EIG is the same in a round
+// and by itself. FP64, 3M splats of which a 384x384 view weighs about a tenth:
+// 94 -> 34 us (at 5, 3 and 2 blocks per SM 37, 38 and 40 us); 60k splats 31 ->
+// 24 us.
+constexpr uint32_t kEigLoads = 4;  // groups of 32 splats whose weights a warp loads together
+template <int MODE, typename Eps>
+__global__ __launch_bounds__(kEigThreads, MODE == SF_EIG_FP64 ? 4 : 5) void eig_kernel(const float* __restrict__ a,
+                                                             const float* __restrict__ b, Eps eps, uint32_t n,
+                                                             const float* __restrict__ table,
+                                                             double* __restrict__ partials,
+                                                             const void* __restrict__ h0) {
     __shared__ double s_warp[kEigThreads / 32];
+    __shared__ uint32_t s_queue[kEigThreads / 32][64];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t lt = (1u << lane) - 1u;
+    uint32_t* queue = s_queue[warp];
+    uint32_t queued = 0;
     double acc = 0.0;
-    const uint32_t stride = gridDim.x * kEigThreads;
-    for (uint32_t i = blockIdx.x * kEigThreads + threadIdx.x; i < n; i += stride) {
-        const float f = fg[i], g = bg ? bg[i] : 0.0f;
-        if (!(f + g > 0.0f)) continue;
-        const float ai = a[i], bi = b[i];
-        if (MODE == SF_EIG_LUT_F32) {
-            const float k = 1.0f + (f + g) / (ai + bi);
-            const float hab = h0 ? static_cast<const float*>(h0)[i] : table_entropy_d(ai, bi, table);
-            const float d = max_(hab - table_entropy_d(ai * k, bi * k, table), 0.0f);
-            acc += (double)d;
-        } else {
-            const double eps = (double)f + (double)g;
-            const double ad = ai, bd = bi;
-            const double k = 1.0 + eps / (ad + bd);
-            const double hab = h0 ? static_cast<const double*>(h0)[i] : beta_entropy_d(ad, bd);
-            const double d = hab - beta_entropy_d(ad * k, bd * k);
-            acc += d > 0.0 ? d : 0.0;
+    const uint64_t stride = (uint64_t)gridDim.x * (kEigThreads * kEigLoads);
+    for (uint64_t base = ((uint64_t)blockIdx.x * (kEigThreads / 32) + warp) * (32 * kEigLoads); base < n;
+         base += stride) {
+        bool live[kEigLoads];
+#pragma unroll
+        for (uint32_t u = 0; u < kEigLoads; ++u) {
+            const uint64_t i = base + u * 32 + lane;
+            live[u] = i < n && eps.any((uint32_t)i);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kEigLoads; ++u) {
+            const uint32_t m = __ballot_sync(0xffffffffu, live[u]);
+            if (live[u]) queue[queued + (uint32_t)__popc(m & lt)] = (uint32_t)base + u * 32 + lane;
+            queued += (uint32_t)__popc(m);
+            __syncwarp();
+            if (queued < 32) continue;
+            const uint32_t i = queue[lane];
+            queued -= 32;
+            const uint32_t rest = lane < queued ? queue[32 + lane] : 0u;
+            __syncwarp();
+            if (lane < queued) queue[lane] = rest;
+            acc += entropy_delta<MODE>(i, eps, a, b, table, h0);
+            __syncwarp();
         }
     }
+    if (lane < queued) acc += entropy_delta<MODE>(queue[lane], eps, a, b, table, h0);
     const double total = block_sum(acc, s_warp);
     if (threadIdx.x == 0) partials[blockIdx.x] = total;
 }
@@ -392,21 +405,34 @@ cudaError_t launch_localize(const float* attr, const float* a, const float* b, u
 }
 
 uint32_t eig_blocks(uint32_t n, int sm_count) {
+    // One splat per thread while that fits the chip: most warps then evaluate
+    // their few live splats in one go.
+    return std::max(1u, std::min((n + kEigThreads - 1) / kEigThreads, (uint32_t)sm_count * 8));
+}
+
+uint32_t localize_blocks(uint32_t n, int sm_count) {
     const uint32_t want = (n + kEigThreads * 4 - 1) / (kEigThreads * 4);
     return std::max(1u, std::min(want, (uint32_t)sm_count * 8));
 }
 
-cudaError_t launch_eig(int mode, const float* a, const float* b, const uint32_t* resp, uint32_t n,
-                       float scale, const float* table, double* partials, uint32_t blocks,
-                       double* out, cudaStream_t stream, const uint32_t* resp2, const void* h0) {
+namespace {
+template <typename Eps>
+cudaError_t eig_go(int mode, const float* a, const float* b, const Eps& eps, uint32_t n, const float* table,
+                   double* partials, uint32_t blocks, double* out, cudaStream_t stream, const void* h0) {
     if (mode == SF_EIG_LUT_F32)
-        eig_kernel<SF_EIG_LUT_F32><<<blocks, kEigThreads, 0, stream>>>(a, b, resp, resp2, n, scale, table, partials,
-                                                                      h0);
+        eig_kernel<SF_EIG_LUT_F32><<<blocks, kEigThreads, 0, stream>>>(a, b, eps, n, table, partials, h0);
     else
-        eig_kernel<SF_EIG_FP64><<<blocks, kEigThreads, 0, stream>>>(a, b, resp, resp2, n, scale, table, partials, h0);
+        eig_kernel<SF_EIG_FP64><<<blocks, kEigThreads, 0, stream>>>(a, b, eps, n, table, partials, h0);
     eig_final_kernel<<<1, kEigThreads, 0, stream>>>(partials, blocks, out);
     note_launches(2);
     return cudaGetLastError();
+}
+}  // namespace
+
+cudaError_t launch_eig(int mode, const float* a, const float* b, const uint32_t* resp, uint32_t n,
+                       float scale, const float* table, double* partials, uint32_t blocks,
+                       double* out, cudaStream_t stream, const uint32_t* resp2, const void* h0) {
+    return eig_go(mode, a, b, EpsWords{resp, resp2, scale}, n, table, partials, blocks, out, stream, h0);
 }
 
 cudaError_t launch_entropy(int mode, const float* a, const float* b, uint32_t n, const float* table, void* out,
@@ -421,13 +447,7 @@ cudaError_t launch_entropy(int mode, const float* a, const float* b, uint32_t n,
 cudaError_t launch_eig_real(int mode, const float* a, const float* b, const float* fg, const float* bg,
                             uint32_t n, const float* table, double* partials, uint32_t blocks, double* out,
                             cudaStream_t stream, const void* h0) {
-    if (mode == SF_EIG_LUT_F32)
-        eig_real_kernel<SF_EIG_LUT_F32><<<blocks, kEigThreads, 0, stream>>>(a, b, fg, bg, n, table, partials, h0);
-    else
-        eig_real_kernel<SF_EIG_FP64><<<blocks, kEigThreads, 0, stream>>>(a, b, fg, bg, n, table, partials, h0);
-    eig_final_kernel<<<1, kEigThreads, 0, stream>>>(partials, blocks, out);
-    note_launches(2);
-    return cudaGetLastError();
+    return eig_go(mode, a, b, EpsReal{fg, bg}, n, table, partials, blocks, out, stream, h0);
 }
 
 cudaError_t launch_beta_update_real(const float* fg, const float* bg, float* a, float* b, uint32_t n,
