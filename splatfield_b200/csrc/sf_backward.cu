@@ -24,14 +24,17 @@
 //  * the geometric adjoints are summed as moments of dL/dpower (dx, dy, dx^2,
 //    dx dy, dy^2; five products per pixel) and turned into the mean's and the
 //    conic's adjoints once per (tile, splat);
-//  * two contributing entries are reduced together, their 16 + 2 values halved
-//    per lane at each step (warp_sum_scatter: 21 shuffles, against 90 for 18
-//    butterfly sums);
+//  * the walked entries are packed two by two (PairRec, last first), so that
+//    powers, exponentials and the products of the adjoints are packed f32
+//    operations and only T and the colour behind go from one to the other;
+//  * the two are reduced together, their 16 + 2 values halved per lane at each
+//    step (warp_sum_scatter: 21 shuffles, against 90 for 18 butterfly sums);
 //  * each warp stores its sums in its own shared slots, marked in a bit mask,
 //    and the flush adds the slots of the warps that have them (shared f32
 //    atomics are compare-and-swap loops).
 // Against the walk of every entry by every warp with nine butterfly sums each:
-// 1M splats at 1080p 1014 -> 425 us, 50k splats at 333x217 329 -> 90 us.
+// 1M splats at 1080p 1014 -> 384 us, 50k splats at 333x217 329 -> 80 us (one
+// entry at a time, contributing ones reduced in pairs: 437 and 90 us).
 // project_bwd_kernel recomputes each splat's projection (src/project.rs:
 // 176-327) and applies the chain rule through conic -> cov2d (det floor,
 // +0.3 dilation), the Jacobian with its 1.3x FOV clamp, R(q) diag(exp s),
@@ -55,14 +58,18 @@ constexpr float C0 = 0.2820948f, C1 = 0.48860252f, C20 = 0.9461747f, C21 = 0.315
 constexpr float K3 = -0.5900436f, A3 = -2.285229f, B3 = 0.4570458f, E3 = 1.8658817f,
                 F3 = 1.119529f, G3 = 1.4453057f;
 
-constexpr uint32_t kBwdChunk = 128;
+// 96 entries a chunk: the stage then takes 54 KB, which with 62 registers a
+// thread leaves four CTAs an SM (128 entries: 67 KB, three, and 397 us where
+// this takes 384 us on 1M splats at 1080p; 64 entries: 388 us).
+constexpr uint32_t kBwdChunk = 96;
 constexpr uint32_t kBwdThreads = 256;
-static_assert(kBwdThreads == 2 * kBwdChunk, "two threads stage and flush one entry");
+static_assert(kBwdThreads >= 2 * kBwdChunk && kBwdChunk % 32 == 0, "two threads stage and flush one entry");
 
 struct BwdStage {
     float4 g0[2][kBwdChunk], g1[2][kBwdChunk], col[2][kBwdChunk];
     float2 ext[2][kBwdChunk];
     uint32_t gid[2][2][kBwdChunk];  // [buffer][staging thread's half][entry]
+    PairRec<true> pairs[kBwdThreads / 32][16];   // the entries a warp replays next
     float part[kBwdThreads / 32][9][kBwdChunk];  // each warp's sums of the chunk
     uint32_t hit[kBwdThreads / 32][kBwdChunk / 32];  // entries it has sums of
     uint32_t max_last;
@@ -104,14 +111,14 @@ __global__ __launch_bounds__(kBwdThreads, 4) void raster_bwd_kernel(BwdArgs a) {
 
     // Threads t and t + kBwdChunk stage entry t of a chunk (the first its
     // geometry, the second its colour) and later flush it (likewise).
-    const uint32_t se = tid & (kBwdChunk - 1u), half = tid / kBwdChunk;
+    const uint32_t se = tid % kBwdChunk, half = tid / kBwdChunk;  // half 2: none
     uint32_t g_next = 0;
     auto load_id = [&](uint32_t c) {
         const uint32_t e = c * kBwdChunk + se;
         g_next = e < max_last ? __ldg(ids + e) : 0u;
     };
     auto issue = [&](uint32_t c, uint32_t b) {
-        if (c * kBwdChunk + se < max_last) {
+        if (half < 2 && c * kBwdChunk + se < max_last) {
             sm.gid[b][half][se] = g_next;
             if (half == 0) {
                 cp_async16(&sm.g0[b][se], a.geo0 + g_next);
@@ -123,7 +130,7 @@ __global__ __launch_bounds__(kBwdThreads, 4) void raster_bwd_kernel(BwdArgs a) {
         }
     };
     auto flush = [&](uint32_t b, uint32_t cnt) {
-        if (se >= cnt) return;
+        if (half >= 2 || se >= cnt) return;
         float v[5] = {0.f, 0.f, 0.f, 0.f, 0.f};
         bool any = false;
 #pragma unroll
@@ -153,16 +160,79 @@ __global__ __launch_bounds__(kBwdThreads, 4) void raster_bwd_kernel(BwdArgs a) {
                 if (v[k] != 0.0f) atomicAdd(dst + 5 + k, v[k]);
         }
     };
-    // Reduces two entries' values (x[8 i + k], k < 8, and y[i] of entry i of
-    // the pair) and stores them; the second may be absent (zeros, jb = ja).
-    auto reduce = [&](float (&x)[16], float (&y)[2], uint32_t ja, uint32_t jb, bool two) {
+    const f32x2 nfx = both(-fx), nfy = both(-fy);
+    PairRec<true>* const recs = sm.pairs[warp];
+    // 1 / (1 - alpha), alpha in [0, 0.999]: the approximate reciprocal and one
+    // Newton-Raphson step (within an ulp of the rounded quotient).
+    auto inv_through = [](float alpha) {
+        const float t = 1.0f - alpha;
+        float r;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(t));
+        return fma_(r, fma_(-t, r, 1.0f), r);
+    };
+    // Replays the two entries of recs[p] (a is the later one) and stores the
+    // warp's sums of their adjoints; `two`: b is an entry. Returns whether
+    // some pixel took one of them. Both entries run through the same
+    // operations whether or not the pixel took them (alpha 0 leaves T as it
+    // is), and where it did not, its terms are selected to zero.
+    auto replay2 = [&](uint32_t p, uint32_t b, uint32_t c0, bool two, uint32_t& ja, uint32_t& jb) -> bool {
+        const float4* r4 = reinterpret_cast<const float4*>(recs + p);
+        const ulonglong2* r = reinterpret_cast<const ulonglong2*>(recs + p);
+        const ulonglong2 xy = r[0], hc = r[1], zo = r[2];
+        const float4 mj = r4[3], rg = r4[4];
+        const float2 bl = *reinterpret_cast<const float2*>(r4 + 5);
+        ja = f2u(mj.z);
+        jb = f2u(mj.w);
+        const f32x2 dx = add2(xy.x, nfx), dy = add2(xy.y, nfy);
+        const f32x2 npow = fma2(mul2(hc.x, dx), dx, fma2(mul2(zo.x, dy), dy, mul2(mul2(hc.y, dx), dy)));
+        float na, nb, oa, ob, ea, eb;
+        exp_neg2(npow, ea, eb);
+        unpack2(npow, na, nb);
+        unpack2(zo.y, oa, ob);
+        const float rawa = oa * ea, rawb = ob * eb;
+        float ala = fminf(rawa, 0.999f), alb = fminf(rawb, 0.999f);
+        const bool oka = c0 + ja < last && ala >= inv255 && !(na < mj.x);
+        const bool okb = c0 + jb < last && alb >= inv255 && !(nb < mj.y);
+        if (!__any_sync(0xffffffffu, oka || okb)) return false;
+        ala = oka ? ala : 0.0f;
+        alb = okb ? alb : 0.0f;
+        // One entry's colour behind it (S) and dL/dalpha, in list order.
+        auto take = [&](bool ok, float alpha, float cr, float cg, float cb, float& w) -> float {
+            const float inv = inv_through(alpha);
+            T *= inv;
+            w = alpha * T;
+            const float er = cr - Sr, eg = cg - Sg, eb2 = cb - Sb;
+            const float dalpha = fma_(T, fma_(g.x, er, fma_(g.y, eg, g.z * eb2)), gw * inv);
+            if (ok) {
+                Sr = fma_(alpha, er, Sr);
+                Sg = fma_(alpha, eg, Sg);
+                Sb = fma_(alpha, eb2, Sb);
+            }
+            return ok ? dalpha : 0.0f;
+        };
+        float wa, wb;
+        float da = take(oka, ala, rg.x, rg.z, bl.x, wa);
+        float db = take(okb, alb, rg.y, rg.w, bl.y, wb);
+        // The clamp at 0.999 passes no gradient to the form and the opacity.
+        da = rawa <= 0.999f ? da : 0.0f;
+        db = rawb <= 0.999f ? db : 0.0f;
+        const f32x2 w2 = pack2(wa, wb), d2 = pack2(da, db);
+        const f32x2 dp = mul2(d2, pack2(-ala, -alb));
+        const f32x2 mx = mul2(dp, dx), my = mul2(dp, dy);
+        const f32x2 v[9] = {mx, my, mul2(mx, dx), mul2(mx, dy), mul2(my, dy), mul2(both(g.x), w2),
+                            mul2(both(g.y), w2), mul2(both(g.z), w2), mul2(d2, pack2(oka ? ea : 0.0f, okb ? eb : 0.0f))};
+        float x[16], y[2];
+#pragma unroll
+        for (uint32_t q = 0; q < 8; ++q) unpack2(v[q], x[q], x[8 + q]);
+        unpack2(v[8], y[0], y[1]);
         warp_sum_scatter(x);
         warp_sum_scatter(y);
-        const uint32_t j = lane < 16 ? ja : jb;
         if (lane < 16 || two) {
+            const uint32_t j = lane < 16 ? ja : jb;
             if (!(lane & 1u)) sm.part[warp][(lane >> 1) & 7u][j] = x[0];
             if ((lane & 15u) == 0) sm.part[warp][8][j] = y[0];
         }
+        return true;
     };
 
     load_id(nch - 1);
@@ -187,73 +257,44 @@ __global__ __launch_bounds__(kBwdThreads, 4) void raster_bwd_kernel(BwdArgs a) {
             uint32_t did = 0;
             if (c0 + (uint32_t)g32 < wlast) {
                 const uint32_t jl = (uint32_t)g32 + lane;
-                const bool reach = c0 + jl < wlast && block_hit(sm.g0[b][jl], sm.g1[b][jl], sm.ext[b][jl], wxf, wyf);
-                uint32_t word = __ballot_sync(0xffffffffu, reach);
-                float x[16], y[2];
-                uint32_t ja = 0;
-                bool pending = false;
-                while (word) {
-                    const uint32_t bit = 31u - (uint32_t)__clz(word);
-                    word ^= 1u << bit;
-                    const uint32_t j = (uint32_t)g32 + bit;
-                    float d[9];
-#pragma unroll
-                    for (uint32_t q = 0; q < 9; ++q) d[q] = 0.0f;
-                    bool hit = false;
-                    const float4 g0 = sm.g0[b][j];
-                    const float4 g1 = sm.g1[b][j];
-                    const float dx = g0.x - fx, dy = g0.y - fy;
-                    const float power = fma_(g0.z * dx, dx, fma_(g1.x * dy, dy, (g0.w * dx) * dy));
-                    if (c0 + j < last && !(power > g1.z)) {
-                        const float G = exp_neg_(-power);
-                        const float raw = g1.y * G;
-                        const float alpha = fminf(raw, 0.999f);
-                        if (alpha >= inv255) {
-                            hit = true;
-                            const float4 c = sm.col[b][j];
-                            const float inv = 1.0f / (1.0f - alpha);
-                            T *= inv;
-                            const float w = alpha * T;
-                            d[5] = g.x * w;
-                            d[6] = g.y * w;
-                            d[7] = g.z * w;
-                            const float er = c.x - Sr, eg = c.y - Sg, eb = c.z - Sb;
-                            const float dalpha = fma_(T, fma_(g.x, er, fma_(g.y, eg, g.z * eb)), gw * inv);
-                            Sr = fma_(alpha, er, Sr);
-                            Sg = fma_(alpha, eg, Sg);
-                            Sb = fma_(alpha, eb, Sb);
-                            if (raw <= 0.999f) {
-                                d[8] = dalpha * G;
-                                const float dp = -dalpha * alpha;
-                                d[0] = dp * dx;
-                                d[1] = dp * dy;
-                                d[2] = d[0] * dx;
-                                d[3] = d[0] * dy;
-                                d[4] = d[1] * dy;
-                            }
-                        }
-                    }
-                    if (!__any_sync(0xffffffffu, hit)) continue;
-                    did |= 1u << bit;
-                    if (!pending) {
-#pragma unroll
-                        for (uint32_t q = 0; q < 8; ++q) x[q] = d[q];
-                        y[0] = d[8];
-                        ja = j;
-                        pending = true;
-                    } else {
-#pragma unroll
-                        for (uint32_t q = 0; q < 8; ++q) x[8 + q] = d[q];
-                        y[1] = d[8];
-                        reduce(x, y, ja, j, true);
-                        pending = false;
-                    }
+                bool reach = c0 + jl < wlast;
+                float4 g0 = make_float4(0.f, 0.f, 0.f, 0.f), g1 = g0;
+                if (reach) {
+                    g0 = sm.g0[b][jl];
+                    g1 = sm.g1[b][jl];
+                    reach = block_hit(g0, g1, sm.ext[b][jl], wxf, wyf);
                 }
-                if (pending) {
-#pragma unroll
-                    for (uint32_t q = 0; q < 8; ++q) x[8 + q] = 0.0f;
-                    y[1] = 0.0f;
-                    reduce(x, y, ja, ja, false);
+                const uint32_t word = __ballot_sync(0xffffffffu, reach);
+                const uint32_t hits = (uint32_t)__popc(word);
+                __syncwarp();  // the last group's records have been read
+                if (reach) {
+                    // Last entry first.
+                    const uint32_t slot = (uint32_t)__popc(word >> lane) - 1u, h = slot & 1u;
+                    PairRec<true>& r = recs[slot >> 1];
+                    const float4 c = sm.col[b][jl];
+                    r.x[h] = g0.x;
+                    r.y[h] = g0.y;
+                    r.nhx[h] = -g0.z;
+                    r.ncy[h] = -g0.w;
+                    r.nhz[h] = -g1.x;
+                    r.op[h] = g1.y;
+                    r.npm[h] = -g1.z;
+                    r.j[h] = jl;
+                    r.r[h] = c.x;
+                    r.g[h] = c.y;
+                    r.b[h] = c.z;
+                }
+                if ((hits & 1u) && lane == 0) {
+                    PairRec<true>& r = recs[hits >> 1];
+                    r.x[1] = r.y[1] = r.nhx[1] = r.ncy[1] = r.nhz[1] = r.op[1] = r.npm[1] = 0.0f;
+                    r.r[1] = r.g[1] = r.b[1] = 0.0f;
+                    r.j[1] = 0u;
+                }
+                __syncwarp();
+                for (uint32_t p = 0; 2 * p < hits; ++p) {
+                    const bool two = 2 * p + 1 < hits;
+                    uint32_t ja, jb;
+                    if (replay2(p, b, c0, two, ja, jb)) did |= (1u << (ja & 31u)) | (two ? 1u << (jb & 31u) : 0u);
                 }
             }
             if (lane == 0) sm.hit[warp][g32 >> 5] = did;

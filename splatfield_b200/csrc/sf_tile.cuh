@@ -1,8 +1,10 @@
 // Device helpers shared by the kernels that walk a tile's list: asynchronous
-// staging copies and the cull tests of a warp's 8x4 pixel block.
+// staging copies, the cull tests of a warp's 8x4 pixel block, packed pairs of
+// entries and warp sums.
 #pragma once
 #include <cstdint>
 #include <cmath>
+#include "sf_math.cuh"
 
 namespace sft {
 
@@ -60,6 +62,68 @@ __device__ __forceinline__ bool block_hit(const float4 g0, const float4 g1, cons
     const float ly = (g0.y - e.y) - wyf, hy = (g0.y + e.y) - wyf;
     if (lx > 7.0f || hx < 0.0f || ly > 3.0f || hy < 0.0f) return false;
     return !block_misses(g0, g1, e, wxf, wyf);
+}
+
+// Two consecutive list entries a and b of a warp's walk, each field of both
+// side by side, so that one 16-byte load fills the operands of two packed f32
+// operations: centres, negated form coefficients and power_max, opacity, the
+// entries' places in the staged chunk and (RGB) colours. The stride (80 or 112
+// bytes) starts the 16 records of a warp in eight different banks.
+template <bool COLOR>
+struct __align__(16) PairRec {
+    float x[2], y[2], nhx[2], ncy[2], nhz[2], op[2], npm[2];
+    uint32_t j[2];
+    float r[COLOR ? 2 : 1], g[COLOR ? 2 : 1], b[COLOR ? 2 : 1];
+    uint32_t pad[COLOR ? 6 : 1];
+};
+static_assert(sizeof(PairRec<true>) == 112 && sizeof(PairRec<false>) == 80, "record stride");
+
+// Packed f32 pairs (sm_100a): each half rounds as the scalar operation does.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v));
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 both(float v) { return pack2(v, v); }
+
+// exp_neg_ (sf_math.cuh) of two values, operation by operation.
+__device__ __forceinline__ void exp_neg2(f32x2 x, float& ea, float& eb) {
+    const f32x2 kr = add2(mul2(x, both(1.44269502f)), both(12582912.0f));
+    const f32x2 kf = add2(kr, both(-12582912.0f));
+    f32x2 r = fma2(kf, both(-0.693145751953125f), x);
+    r = fma2(kf, both(-1.42860677e-06f), r);
+    f32x2 p = both(1.98412701e-04f);
+    p = fma2(p, r, both(1.38888892e-03f));
+    p = fma2(p, r, both(8.33333377e-03f));
+    p = fma2(p, r, both(4.16666679e-02f));
+    p = fma2(p, r, both(1.66666672e-01f));
+    p = fma2(p, r, both(0.5f));
+    p = fma2(p, r, both(1.0f));
+    p = fma2(p, r, both(1.0f));
+    float pa, pb, ka, kb;
+    unpack2(p, pa, pb);
+    unpack2(kr, ka, kb);
+    ea = sfm::u2f(sfm::f2u(pa) + (sfm::f2u(ka) << 23));
+    eb = sfm::u2f(sfm::f2u(pb) + (sfm::f2u(kb) << 23));
 }
 
 // Sums N = 2^k values over the warp's lanes at once, halving the values held
