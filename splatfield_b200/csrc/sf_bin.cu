@@ -156,6 +156,9 @@ struct ClassLimits {
     uint32_t max_n[kSortClasses - 1];  // longest list of each class but the last
 };
 
+// A thread's share of the chunks (chunks <= 32 kColChunks: 2 per SM).
+constexpr uint32_t kColChunks = 12;
+
 // Block (32, 32): x = tile within the block's 32, y = a group of chunks.
 // words: [6] max tile count (atomicMax), [8 + k] tiles in size class k
 // (lists[k * tiles + i]); class kSortClasses - 1 holds the lists longer than
@@ -167,54 +170,66 @@ __global__ __launch_bounds__(1024) void bin_colscan_kernel(uint32_t* __restrict_
     pdl_trigger();
     pdl_wait();
     __shared__ uint32_t s_part[32][33];
+    __shared__ uint32_t s_total[32];
     const uint32_t tx = threadIdx.x, ty = threadIdx.y;
     const uint32_t t = blockIdx.x * 32u + tx;
     const bool valid = t < tiles;
     const uint32_t per = (chunks + 31u) / 32u;
     const uint32_t c0 = min(chunks, ty * per), c1 = min(chunks, c0 + per);
+    // This thread's counts (all loads in flight together), kept for the second
+    // half.
+    uint32_t v[kColChunks];
     uint32_t sum = 0;
-    if (valid)
-        for (uint32_t c = c0; c < c1; ++c) sum += hist[(size_t)c * tiles + t];
+#pragma unroll
+    for (uint32_t k = 0; k < kColChunks; ++k)
+        v[k] = valid && c0 + k < c1 ? hist[(size_t)(c0 + k) * tiles + t] : 0u;
+#pragma unroll
+    for (uint32_t k = 0; k < kColChunks; ++k) sum += v[k];
     s_part[ty][tx] = sum;
     __syncthreads();
-    if (ty == 0) {
-        uint32_t run = 0;
-        for (uint32_t y = 0; y < 32; ++y) {
-            const uint32_t v = s_part[y][tx];
-            s_part[y][tx] = run;
-            run += v;
+    // Warp y turns tile y's 32 group sums into their prefix.
+    {
+        const uint32_t g = s_part[tx][ty];
+        uint32_t incl = g;
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const uint32_t x = __shfl_up_sync(0xffffffffu, incl, d);
+            if (tx >= d) incl += x;
         }
-        if (valid) cnt[t] = run;
+        s_part[tx][ty] = incl - g;
+        if (tx == 31) s_total[ty] = incl;
+    }
+    __syncthreads();
+    uint32_t run = s_part[ty][tx];
+#pragma unroll
+    for (uint32_t k = 0; k < kColChunks; ++k) {
+        if (valid && c0 + k < c1) hist[(size_t)(c0 + k) * tiles + t] = run;
+        run += v[k];
+    }
+    if (ty == 0) {
+        const uint32_t total = valid ? s_total[tx] : 0u;
+        if (valid) cnt[t] = total;
         if (blockIdx.x == 0 && tx == 0) cnt[tiles] = 0;
-        // Size classes (warp-aggregated appends; the list order is free).
-        const uint32_t total = valid ? run : 0u;
+        // Size classes (warp-aggregated appends; the list order is free): lane
+        // k takes class k's slots, so the eight counters cost one round trip.
         uint32_t cls = total == 0 ? kSortClasses : kSortClasses - 1;  // kSortClasses: the empty tiles
         if (total > 0)
             for (int k = kSortClasses - 2; k >= 0; --k)
                 if (total <= lim.max_n[k]) cls = (uint32_t)k;
         const uint32_t mx = __reduce_max_sync(0xffffffffu, total);
         if (tx == 0 && mx) atomicMax(words + 6, mx);
+        uint32_t mine = 0, peers = 0;
 #pragma unroll
         for (uint32_t k = 0; k <= kSortClasses; ++k) {
-            const uint32_t m = __ballot_sync(0xffffffffu, valid && cls == k);
-            if (!m) continue;
-            const uint32_t leader = __ffs(m) - 1;
-            uint32_t base = 0;
-            if (tx == leader) base = atomicAdd(words + 8u + k, __popc(m));
-            base = __shfl_sync(0xffffffffu, base, leader);
             // Lanes past the last tile are of the empty class too: not filed.
-            if (valid && cls == k) lists[k * tiles + base + __popc(m & lanemask_lt())] = t;
+            const uint32_t m = __ballot_sync(0xffffffffu, valid && cls == k);
+            if (tx == k) mine = (uint32_t)__popc(m);
+            if (cls == k) peers = m;
         }
-    }
-    __syncthreads();
-    if (valid) {
-        uint32_t run = s_part[ty][tx];
-        for (uint32_t c = c0; c < c1; ++c) {
-            const size_t i = (size_t)c * tiles + t;
-            const uint32_t v = hist[i];
-            hist[i] = run;
-            run += v;
-        }
+        uint32_t base = 0;
+        if (mine) base = atomicAdd(words + 8u + tx, mine);
+        base = __shfl_sync(0xffffffffu, base, cls);
+        if (valid) lists[cls * tiles + base + __popc(peers & lanemask_lt())] = t;
     }
 }
 
@@ -1169,7 +1184,7 @@ cudaError_t smem_opt_in(const void* fn, size_t smem) {
 // column scan and place 14.4 -> 13.6 us).
 constexpr uint32_t kMinBinChunk = 512;
 uint32_t bin_chunks(uint32_t n, int sm_count) {
-    const uint32_t c = (uint32_t)std::max(1, 2 * sm_count);
+    const uint32_t c = std::min((uint32_t)std::max(1, 2 * sm_count), 32 * kColChunks);
     return std::max(1u, std::min(c, (n + kMinBinChunk - 1) / kMinBinChunk));
 }
 
