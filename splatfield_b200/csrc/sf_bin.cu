@@ -39,17 +39,85 @@ __device__ __forceinline__ uint32_t lanemask_lt() {
     return m;
 }
 
+// Calls f(lane, tile, payload) for every tile of the boxes bb of a warp's 32
+// splats (packed min / max tile; an empty box has no pairs; pay: a word of the
+// lane's splat). The pairs are handed to the lanes in turn (owner found by a
+// shuffle search over the lanes' inclusive ends), so a splat covering many
+// tiles does not stall its warp. U rounds of 32 pairs are handed out per step:
+// their searches and f calls are independent, so their shuffle and
+// shared-memory latencies overlap. Every lane of the warp calls it. pairs
+// (optional): += this lane's splat's pairs.
+template <uint32_t U, typename F>
+__device__ __forceinline__ void spread_pairs(const uint2 bb, const uint32_t pay, uint32_t tiles_x, F&& f,
+                                             unsigned long long* pairs = nullptr) {
+    const uint32_t lane = threadIdx.x & 31u;
+            uint32_t min_x = bb.x & 0xffffu, min_y = bb.x >> 16, width = 1, cnt = 0;
+            const uint32_t max_x = bb.y & 0xffffu, max_y = bb.y >> 16;
+            if (max_x > min_x && max_y > min_y) {
+                width = max_x - min_x;
+                cnt = width * (max_y - min_y);
+            }
+            if (pairs) *pairs += cnt;
+            // 1 / width, shuffled to the pair lanes with the box.
+            const float rw = __fdividef(1.0f, (float)width);
+            uint32_t incl = cnt;
+    #pragma unroll
+            for (uint32_t d = 1; d < 32; d <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += v;
+            }
+            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+            for (uint32_t p0 = 0; p0 < total; p0 += 32u * U) {
+                uint32_t o[U];
+    #pragma unroll
+                for (uint32_t u = 0; u < U; ++u) o[u] = 0;
+    #pragma unroll
+                for (uint32_t step = 16; step > 0; step >>= 1) {
+    #pragma unroll
+                    for (uint32_t u = 0; u < U; ++u) {
+                        const uint32_t v = __shfl_sync(0xffffffffu, incl, o[u] + step - 1);
+                        if (v <= p0 + 32u * u + lane) o[u] += step;
+                    }
+                }
+    #pragma unroll
+                for (uint32_t u = 0; u < U; ++u) {
+                    const uint32_t p = p0 + 32u * u + lane;
+                    const uint32_t oend = __shfl_sync(0xffffffffu, incl, o[u]);
+                    const uint32_t ocnt = __shfl_sync(0xffffffffu, cnt, o[u]);
+                    const uint32_t ow = __shfl_sync(0xffffffffu, width, o[u]);
+                    const float orw = __shfl_sync(0xffffffffu, rw, o[u]);
+                    const uint32_t ox = __shfl_sync(0xffffffffu, min_x, o[u]);
+                    const uint32_t oy = __shfl_sync(0xffffffffu, min_y, o[u]);
+                    const uint32_t opay = __shfl_sync(0xffffffffu, pay, o[u]);
+                    if (p < total) {
+                        // Row and column of pair k in the owner's box: a float
+                        // quotient (k < 2^16, so it is off by at most one) and an
+                        // exact integer correction.
+                        const uint32_t k = p - (oend - ocnt);
+                        uint32_t row = (uint32_t)((float)k * orw);
+                        int32_t col = (int32_t)(k - row * ow);
+                        if (col < 0) {
+                            --row;
+                            col += (int32_t)ow;
+                        } else if (col >= (int32_t)ow) {
+                            ++row;
+                            col -= (int32_t)ow;
+                        }
+                        f(o[u], (ox + (uint32_t)col) + (oy + row) * tiles_x, opay);
+                    }
+                }
+            }
+}
+
 // Calls f(splat, tile, payload) for every tile of every splat in [begin,
-// end): warps take 32 consecutive splats at a time and spread the pairs over
-// their lanes (owner found by a shuffle search over the lanes' inclusive
-// ends), so a splat covering many tiles does not stall its warp. payload
-// (optional) is a per-splat word loaded once by the splat's lane with its box
-// and shuffled to the lanes that emit its pairs. U rounds of 32 pairs are
-// handed out per step: their searches and f calls are independent, so their
-// shuffle and shared-memory latencies overlap.
+// end): warps take 32 consecutive splats at a time and spread their pairs over
+// their lanes. payload (optional) is a per-splat word loaded once by the
+// splat's lane with its box.
+// pairs (optional): += this lane's splats' pairs.
 template <uint32_t U, typename F>
 __device__ __forceinline__ void for_each_pair(uint32_t begin, uint32_t end, const uint2* __restrict__ bbox,
-                                              const uint32_t* __restrict__ payload, uint32_t tiles_x, F&& f) {
+                                              const uint32_t* __restrict__ payload, uint32_t tiles_x, F&& f,
+                                              unsigned long long* pairs = nullptr) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t stride = (blockDim.x >> 5) * 32u;
@@ -72,61 +140,7 @@ __device__ __forceinline__ void for_each_pair(uint32_t begin, uint32_t end, cons
             bb_next = bbox[rn];
             if (payload) pay_next = payload[rn];
         }
-        uint32_t min_x = bb.x & 0xffffu, min_y = bb.x >> 16, width = 1, cnt = 0;
-        const uint32_t max_x = bb.y & 0xffffu, max_y = bb.y >> 16;
-        if (max_x > min_x && max_y > min_y) {
-            width = max_x - min_x;
-            cnt = width * (max_y - min_y);
-        }
-        // 1 / width, shuffled to the pair lanes with the box.
-        const float rw = __fdividef(1.0f, (float)width);
-        uint32_t incl = cnt;
-#pragma unroll
-        for (uint32_t d = 1; d < 32; d <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-            if (lane >= d) incl += v;
-        }
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        for (uint32_t p0 = 0; p0 < total; p0 += 32u * U) {
-            uint32_t o[U];
-#pragma unroll
-            for (uint32_t u = 0; u < U; ++u) o[u] = 0;
-#pragma unroll
-            for (uint32_t step = 16; step > 0; step >>= 1) {
-#pragma unroll
-                for (uint32_t u = 0; u < U; ++u) {
-                    const uint32_t v = __shfl_sync(0xffffffffu, incl, o[u] + step - 1);
-                    if (v <= p0 + 32u * u + lane) o[u] += step;
-                }
-            }
-#pragma unroll
-            for (uint32_t u = 0; u < U; ++u) {
-                const uint32_t p = p0 + 32u * u + lane;
-                const uint32_t oend = __shfl_sync(0xffffffffu, incl, o[u]);
-                const uint32_t ocnt = __shfl_sync(0xffffffffu, cnt, o[u]);
-                const uint32_t ow = __shfl_sync(0xffffffffu, width, o[u]);
-                const float orw = __shfl_sync(0xffffffffu, rw, o[u]);
-                const uint32_t ox = __shfl_sync(0xffffffffu, min_x, o[u]);
-                const uint32_t oy = __shfl_sync(0xffffffffu, min_y, o[u]);
-                const uint32_t opay = __shfl_sync(0xffffffffu, pay, o[u]);
-                if (p < total) {
-                    // Row and column of pair k in the owner's box: a float
-                    // quotient (k < 2^16, so it is off by at most one) and an
-                    // exact integer correction.
-                    const uint32_t k = p - (oend - ocnt);
-                    uint32_t row = (uint32_t)((float)k * orw);
-                    int32_t col = (int32_t)(k - row * ow);
-                    if (col < 0) {
-                        --row;
-                        col += (int32_t)ow;
-                    } else if (col >= (int32_t)ow) {
-                        ++row;
-                        col -= (int32_t)ow;
-                    }
-                    f(g0 + o[u], (ox + (uint32_t)col) + (oy + row) * tiles_x, opay);
-                }
-            }
-        }
+        spread_pairs<U>(bb, pay, tiles_x, [&](uint32_t l, uint32_t t, uint32_t p) { f(g0 + l, t, p); }, pairs);
     }
 }
 
@@ -255,6 +269,257 @@ __global__ __launch_bounds__(kBinThreads) void bin_place_kernel(
         }
     });
     if (over) atomicOr(err, SF_DEV_ERR_CAPACITY);
+}
+
+// Block-wide exclusive scan of one value per thread; s32 holds 32 words.
+// Returns the exclusive prefix; total gets the sum (uniform).
+template <uint32_t THREADS>
+__device__ __forceinline__ uint32_t block_scan(uint32_t x, uint32_t* s32, uint32_t& total) {
+    constexpr uint32_t WARPS = THREADS / 32;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t incl = x;
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+    }
+    __syncthreads();
+    if (lane == 31) s32[warp] = incl;
+    __syncthreads();
+    uint32_t wbase = 0, tot = 0;
+    for (uint32_t w = 0; w < WARPS; ++w) {
+        const uint32_t v = s32[w];
+        if (w < warp) wbase += v;
+        tot += v;
+    }
+    total = tot;
+    return wbase + incl - x;
+}
+
+// ---- depth-limited lists
+//
+// A tile's pixels are saturated after its first few hundred entries: the
+// raster of a 512x512 view of 1M splats walks 5 to 8% of its pairs, but all of
+// them are placed and sorted. So a round's view places heads only:
+//   1. head_sample: the depth keys of every eighth splat, per tile;
+//   2. head_pick: per tile the key below which about kHeadTarget of its pairs
+//      lie (tiles whose whole list is about that short get no limit);
+//   3. count, place, sorts and raster over the pairs up to the limit. A tile
+//      with a pixel not saturated by its head is listed, and the pixels'
+//      transmittances are kept;
+//   4. tail_count, tail_plan, tail_place: the listed tiles' other pairs, found
+//      by testing every splat's box against a bit per tile; the raster orders
+//      and composites them from the kept transmittances (raster_tails_kernel).
+// Heads end at a key, so head and tail are the sorted list cut in two, and the
+// pixels take the same entries in the same order: the words are the same. A
+// limit is only a guess; a bad one costs time.
+//
+// Measured (whole rounds, with whole lists -> with heads): 20 masked 512x512
+// views of 1M splats 2.88 -> 2.64 ms; 16 views of 256 to 1024 squared of 3M
+// 7.18 -> 5.32 ms; 12 views of 1024 squared of 3M 7.24 -> 4.50 ms and of 2.2M
+// 8.55 -> 4.90 ms. Heads of 1024, 1536, 2048 and 3072 pairs: 2.68, 2.57, 2.64
+// and 2.70 ms on the first, 6.76, 6.65, 6.25 and 6.34 ms on the second (small
+// views included). Where the lists are short or the tiles few, the six more
+// kernels of a view are not repaid: 12 views of 512 squared of 530k splats
+// 1.19 -> 1.21 ms, of 256 squared of 300k 0.93 -> 1.20 ms, of 200 squared of
+// 1M 2.27 -> 3.05 ms; hence heads_wanted.
+constexpr uint32_t kHeadStride = 32;     // splats per sampled splat
+static_assert(kHeadStride == 32, "the sample's place is five bits");
+constexpr uint32_t kHeadTarget = 2048;   // pairs aimed at
+constexpr uint32_t kHeadKeep = 3072;     // lists estimated no longer than this are not cut
+constexpr uint32_t kHeadMinSplats = 640000, kHeadMinTiles = 1024, kHeadSplats = 512;
+constexpr uint32_t kHeadMaxTiles = 12288;  // limits and counters of a block: 96 KB
+
+__global__ __launch_bounds__(256) void head_sample_kernel(const uint2* __restrict__ bbox,
+                                                          const uint32_t* __restrict__ depth_keys, uint32_t n,
+                                                          uint32_t tiles_x, HeadState h) {
+    const uint32_t k = blockIdx.x * 256u + threadIdx.x;
+    // One of each kHeadStride neighbours, at a place that varies.
+    const uint64_t i = (uint64_t)k * kHeadStride + ((k * 2654435761u) >> 27);
+    uint2 bb = make_uint2(0u, 0u);
+    uint32_t key = 0;
+    if (i < n) {
+        bb = bbox[i];
+        key = depth_keys[i];
+    }
+    spread_pairs<1>(bb, key, tiles_x, [&](uint32_t, uint32_t t, uint32_t kk) {
+        const uint32_t slot = atomicAdd(h.sampled + 8 * (size_t)t, 1u);
+        if (slot < kHeadSamples) h.keys[(size_t)t * kHeadSamples + slot] = kk;
+    });
+}
+
+// A warp per tile: the rank-th smallest of its sampled keys, by bisection.
+__global__ __launch_bounds__(256) void head_pick_kernel(uint32_t tiles, HeadState h) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t t = blockIdx.x * 8u + (threadIdx.x >> 5);
+    if (t >= tiles) return;
+    const uint32_t c = h.sampled[8 * (size_t)t];
+    uint32_t limit = 0xffffffffu;
+    if (c > kHeadKeep / kHeadStride) {
+        const uint32_t m = min(c, kHeadSamples);
+        const uint32_t rank = max(1u, kHeadTarget / kHeadStride * m / c);
+        uint32_t k[kHeadSamples / 32];
+        uint32_t lo = 0xffffffffu, hi = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < kHeadSamples / 32; ++j) {
+            k[j] = j * 32 + lane < m ? h.keys[(size_t)t * kHeadSamples + j * 32 + lane] : 0xffffffffu;
+            if (j * 32 + lane < m) {
+                lo = min(lo, k[j]);
+                hi = max(hi, k[j]);
+            }
+        }
+        lo = __reduce_min_sync(0xffffffffu, lo);
+        hi = __reduce_max_sync(0xffffffffu, hi);
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            uint32_t below = 0;
+#pragma unroll
+            for (uint32_t j = 0; j < kHeadSamples / 32; ++j) below += j * 32 + lane < m && k[j] <= mid;
+            if (__reduce_add_sync(0xffffffffu, below) >= rank) hi = mid;
+            else lo = mid + 1;
+        }
+        limit = lo;
+    }
+    if (lane == 0) h.limit[t] = limit;
+}
+
+__global__ __launch_bounds__(kBinThreads, 2) void head_count_kernel(
+    const uint2* __restrict__ bbox, const uint32_t* __restrict__ depth_keys, uint32_t n, uint32_t chunk,
+    uint32_t tiles_x, uint32_t tiles, uint32_t* __restrict__ hist, const uint32_t* __restrict__ limit,
+    unsigned long long* total_all) {
+    extern __shared__ uint32_t s_hist[];
+    uint32_t* s_limit = s_hist + tiles;
+    for (uint32_t t = threadIdx.x; t < tiles; t += blockDim.x) {
+        s_hist[t] = 0;
+        s_limit[t] = limit[t];
+    }
+    __syncthreads();
+    const uint32_t begin = min(n, blockIdx.x * chunk);
+    const uint32_t end = min(n, begin + chunk);
+    unsigned long long all = 0;
+    for_each_pair<kCountUnroll>(begin, end, bbox, depth_keys, tiles_x, [&](uint32_t, uint32_t t, uint32_t key) {
+        if (key <= s_limit[t]) atomicAdd(&s_hist[t], 1u);
+    }, &all);
+    for (uint32_t d = 16; d > 0; d >>= 1) all += __shfl_xor_sync(0xffffffffu, all, d);
+    if ((threadIdx.x & 31u) == 0 && all) atomicAdd(total_all, all);
+    __syncthreads();
+    uint32_t* row = hist + (size_t)blockIdx.x * tiles;
+    for (uint32_t t = threadIdx.x; t < tiles; t += blockDim.x) row[t] = s_hist[t];
+}
+
+__global__ __launch_bounds__(kBinThreads) void head_place_kernel(
+    const uint2* __restrict__ bbox, const uint32_t* __restrict__ depth_keys, uint32_t n, uint32_t chunk,
+    uint32_t tiles_x, uint32_t tiles, const uint32_t* __restrict__ hist, const uint32_t* __restrict__ tile_start,
+    uint32_t capacity, uint2* __restrict__ pairs, uint32_t* err, const uint32_t* __restrict__ limit) {
+    pdl_trigger();
+    pdl_wait();
+    extern __shared__ uint32_t s_cur[];
+    uint32_t* s_limit = s_cur + tiles;
+    const uint32_t* row = hist + (size_t)blockIdx.x * tiles;
+    for (uint32_t t = threadIdx.x; t < tiles; t += blockDim.x) {
+        s_cur[t] = tile_start[t] + row[t];
+        s_limit[t] = limit[t];
+    }
+    __syncthreads();
+    const uint32_t begin = min(n, blockIdx.x * chunk);
+    const uint32_t end = min(n, begin + chunk);
+    bool over = false;
+    for_each_pair<kPlaceUnroll>(begin, end, bbox, depth_keys, tiles_x, [&](uint32_t s, uint32_t t, uint32_t key) {
+        if (key > s_limit[t]) return;
+        const uint32_t slot = atomicAdd(&s_cur[t], 1u);
+        if (slot < capacity) {
+            pairs[slot] = make_uint2(key, s);
+        } else {
+            over = true;
+        }
+    });
+    if (over) atomicOr(err, SF_DEV_ERR_CAPACITY);
+}
+
+// Calls f(tile, key, splat) for the tail pairs of the listed tiles (s_bits: the
+// listed tiles, a bit each). A thread per splat; most boxes meet no listed tile.
+template <typename F>
+__device__ __forceinline__ void for_each_tail_pair(const uint2* __restrict__ bbox,
+                                                   const uint32_t* __restrict__ depth_keys, uint32_t n,
+                                                   uint32_t tiles_x, const uint32_t* s_bits,
+                                                   const uint32_t* __restrict__ limit, F&& f) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint2 bb = bbox[i];
+        for (uint32_t y = bb.x >> 16; y < (bb.y >> 16); ++y)
+            for (uint32_t x = bb.x & 0xffffu; x < (bb.y & 0xffffu); ++x) {
+                const uint32_t t = x + y * tiles_x;
+                if (!((s_bits[t >> 5] >> (t & 31u)) & 1u)) continue;
+                const uint32_t key = depth_keys[i];
+                if (key > limit[t]) f(t, key, i);
+            }
+    }
+}
+
+// Counts and slots go through a counter per tile in shared memory: a listed
+// tile's tail may hold thousands of pairs, and as many atomics on one address.
+constexpr uint32_t kTailThreads = 512;
+__global__ __launch_bounds__(kTailThreads) void tail_count_kernel(const uint2* __restrict__ bbox,
+                                                                  const uint32_t* __restrict__ depth_keys, uint32_t n,
+                                                                  uint32_t tiles_x, uint32_t tiles, HeadState h) {
+    if (h.ctrl[0] == 0) return;
+    extern __shared__ uint32_t s_n[];
+    __shared__ uint32_t s_bits[kHeadMaxTiles / 32];
+    for (uint32_t w = threadIdx.x; w < (tiles + 31) / 32; w += kTailThreads) s_bits[w] = h.bits[w];
+    for (uint32_t t = threadIdx.x; t < tiles; t += kTailThreads) s_n[t] = 0;
+    __syncthreads();
+    for_each_tail_pair(bbox, depth_keys, n, tiles_x, s_bits, h.limit,
+                       [&](uint32_t t, uint32_t, uint32_t) { atomicAdd(s_n + t, 1u); });
+    __syncthreads();
+    for (uint32_t t = threadIdx.x; t < tiles; t += kTailThreads)
+        if (s_n[t]) atomicAdd(h.tail_n + t, s_n[t]);
+}
+
+// First slots of the listed tiles' tails, after the heads.
+// *listed = how many they are.
+__global__ __launch_bounds__(1024) void tail_plan_kernel(HeadState h, uint32_t capacity, uint32_t* listed) {
+    __shared__ uint32_t s32[32];
+    const uint32_t count = h.ctrl[0];
+    if (threadIdx.x == 0) *listed = count;
+    const unsigned long long heads = *reinterpret_cast<const unsigned long long*>(h.ctrl + 2);
+    uint32_t base = (uint32_t)(heads < capacity ? heads : capacity);
+    for (uint32_t i0 = 0; i0 < count; i0 += 1024) {
+        const uint32_t i = i0 + threadIdx.x;
+        const uint32_t t = i < count ? h.list[i] : 0u;
+        const uint32_t c = i < count ? h.tail_n[t] : 0u;
+        uint32_t total;
+        const uint32_t at = base + block_scan<1024>(c, s32, total);
+        if (i < count) {
+            // Past the capacity the frame is drawn again after it has grown.
+            h.tail_start[t] = h.tail_at[t] = min(at, capacity);
+            h.tail_n[t] = at < capacity ? min(c, capacity - at) : 0u;
+        }
+        base += total;
+    }
+}
+
+__global__ __launch_bounds__(kTailThreads) void tail_place_kernel(const uint2* __restrict__ bbox,
+                                                                  const uint32_t* __restrict__ depth_keys, uint32_t n,
+                                                                  uint32_t tiles_x, uint32_t tiles, uint32_t capacity,
+                                                                  uint2* __restrict__ pairs, uint32_t* err,
+                                                                  HeadState h) {
+    if (h.ctrl[0] == 0) return;
+    extern __shared__ uint32_t s_n[];
+    __shared__ uint32_t s_bits[kHeadMaxTiles / 32];
+    for (uint32_t w = threadIdx.x; w < (tiles + 31) / 32; w += kTailThreads) s_bits[w] = h.bits[w];
+    for (uint32_t t = threadIdx.x; t < tiles; t += kTailThreads) s_n[t] = 0;
+    __syncthreads();
+    for_each_tail_pair(bbox, depth_keys, n, tiles_x, s_bits, h.limit,
+                       [&](uint32_t t, uint32_t, uint32_t) { atomicAdd(s_n + t, 1u); });
+    __syncthreads();
+    // This block's slots of each tail.
+    for (uint32_t t = threadIdx.x; t < tiles; t += kTailThreads)
+        if (s_n[t]) s_n[t] = atomicAdd(h.tail_at + t, s_n[t]);
+    __syncthreads();
+    for_each_tail_pair(bbox, depth_keys, n, tiles_x, s_bits, h.limit, [&](uint32_t t, uint32_t key, uint32_t s) {
+        const uint32_t slot = atomicAdd(s_n + t, 1u);
+        if (slot < capacity) pairs[slot] = make_uint2(key, s);
+        else atomicOr(err, SF_DEV_ERR_CAPACITY);
+    });
 }
 
 // ---- per-tile sort
@@ -868,31 +1133,6 @@ __device__ __forceinline__ uint32_t giant_bucket(uint32_t k, uint32_t mn, uint32
     return min((k - mn) >> shift, kGiantBins - 1);
 }
 
-// Block-wide exclusive scan of one value per thread; s32 holds 32 words.
-// Returns the exclusive prefix; total gets the sum (uniform).
-template <uint32_t THREADS>
-__device__ __forceinline__ uint32_t block_scan(uint32_t x, uint32_t* s32, uint32_t& total) {
-    constexpr uint32_t WARPS = THREADS / 32;
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t incl = x;
-#pragma unroll
-    for (uint32_t d = 1; d < 32; d <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += v;
-    }
-    __syncthreads();
-    if (lane == 31) s32[warp] = incl;
-    __syncthreads();
-    uint32_t wbase = 0, tot = 0;
-    for (uint32_t w = 0; w < WARPS; ++w) {
-        const uint32_t v = s32[w];
-        if (w < warp) wbase += v;
-        tot += v;
-    }
-    total = tot;
-    return wbase + incl - x;
-}
-
 __global__ __launch_bounds__(1024) void giant_select_kernel(const uint32_t* __restrict__ list, const uint32_t* list_n,
                                                             const uint32_t* __restrict__ tile_start,
                                                             uint32_t capacity, GiantState gs) {
@@ -1172,7 +1412,7 @@ cudaError_t launch_sort_kernel(K kernel, uint32_t threads, size_t smem, uint32_t
 }
 
 cudaError_t smem_opt_in(const void* fn, size_t smem) {
-    if (smem <= 48 * 1024) return cudaSuccess;
+    if (smem <= 40 * 1024) return cudaSuccess;
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 }
 
@@ -1239,6 +1479,59 @@ cudaError_t launch_bin_place(const uint2* bbox, const uint32_t* depth_keys, uint
                    tiles_x, tiles, hist, tile_start, capacity, pairs, err);
     note_launches(1);
     return e;
+}
+
+bool heads_wanted(uint32_t n, uint32_t tiles) {
+    return n >= kHeadMinSplats && tiles >= kHeadMinTiles && tiles <= kHeadMaxTiles && n / kHeadSplats >= tiles;
+}
+
+cudaError_t launch_head_limits(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
+                               uint32_t tiles, const HeadState& h, cudaStream_t st) {
+    const uint32_t sampled = (n + kHeadStride - 1) / kHeadStride;
+    head_sample_kernel<<<(sampled + 255) / 256, 256, 0, st>>>(bbox, depth_keys, n, tiles_x, h);
+    head_pick_kernel<<<(tiles + 7) / 8, 256, 0, st>>>(tiles, h);
+    note_launches(2);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_head_count(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
+                              uint32_t tiles, uint32_t chunks, uint32_t* hist, const HeadState& h,
+                              unsigned long long* total_all, cudaStream_t st) {
+    const size_t smem = (size_t)tiles * 8;
+    const cudaError_t e = smem_opt_in((const void*)head_count_kernel, smem);
+    if (e != cudaSuccess) return e;
+    head_count_kernel<<<chunks, kBinThreads, smem, st>>>(bbox, depth_keys, n, bin_chunk_size(n, chunks), tiles_x, tiles,
+                                                         hist, h.limit, total_all);
+    note_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_head_place(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
+                              uint32_t tiles, uint32_t chunks, const uint32_t* hist, const uint32_t* tile_start,
+                              uint32_t capacity, uint2* pairs, uint32_t* err, const HeadState& h, cudaStream_t st) {
+    const size_t smem = (size_t)tiles * 8;
+    cudaError_t e = smem_opt_in((const void*)head_place_kernel, smem);
+    if (e != cudaSuccess) return e;
+    e = launch_pdl(head_place_kernel, chunks, kBinThreads, smem, st, bbox, depth_keys, n, bin_chunk_size(n, chunks),
+                   tiles_x, tiles, hist, tile_start, capacity, pairs, err, (const uint32_t*)h.limit);
+    note_launches(1);
+    return e;
+}
+
+cudaError_t launch_tail_place(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
+                              uint32_t tiles, uint32_t capacity, uint2* pairs, uint32_t* words, const HeadState& h,
+                              cudaStream_t st) {
+    const uint32_t blocks = std::min((n + kTailThreads - 1) / kTailThreads, 296u);
+    const size_t smem = (size_t)tiles * 4;
+    cudaError_t e = smem_opt_in((const void*)tail_count_kernel, smem);
+    if (e == cudaSuccess) e = smem_opt_in((const void*)tail_place_kernel, smem);
+    if (e != cudaSuccess) return e;
+    tail_count_kernel<<<blocks, kTailThreads, smem, st>>>(bbox, depth_keys, n, tiles_x, tiles, h);
+    tail_plan_kernel<<<1, 1024, 0, st>>>(h, capacity, words + 3);
+    tail_place_kernel<<<blocks, kTailThreads, smem, st>>>(bbox, depth_keys, n, tiles_x, tiles, capacity, pairs, words + 1,
+                                                          h);
+    note_launches(3);
+    return cudaGetLastError();
 }
 
 namespace {

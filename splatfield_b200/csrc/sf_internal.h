@@ -128,7 +128,19 @@ struct RasterArgs {
     // class_n[k], k = kSortClasses - 1 .. 0, then the empty tiles).
     const uint32_t* class_lists;
     const uint32_t* class_n;
+    // Depth-limited lists (optional, modes 1 to 3): the lists are heads; tiles
+    // with a tail that some pixel is not saturated before are listed.
+    const uint32_t* head_limit;
+    uint32_t* head_ctrl;
+    uint32_t* head_bits;
+    uint32_t* head_list;
+    float* head_t;
+    const uint32_t* tail_start;
+    const uint32_t* tail_n;
 };
+// The listed tiles' tails (unsorted pairs from tail_start, tail_n of them),
+// taken up from head_t; args as for the heads, with `pairs`.
+cudaError_t launch_raster_tails(int mode, const RasterArgs& a, int sm_count, cudaStream_t stream);
 // mode 0 = RGB, 1 = total responsibility, 2 = evidence, 3 = real-valued fg /
 // bg responsibilities (afg[i] += sum_p mask(p) alpha_i T_i(p), abg[i] += sum_p
 // (1 - mask(p)) alpha_i T_i(p); mask null: all in afg). ext is always needed.
@@ -205,6 +217,44 @@ constexpr uint32_t kBinSharedMax = 12288;
 // (all zero on entry).
 cudaError_t launch_bin_count(const uint2* bbox, uint32_t n, uint32_t tiles_x, uint32_t tiles, uint32_t chunks,
                              uint32_t* hist, cudaStream_t st);
+// Depth-limited lists of a round's view (sf_bin.cu): the nearest pairs of each
+// tile (its head, up to a depth key `limit` picked from a sample of the
+// splats) are placed, sorted and rasterized; a tile that some pixel walks past
+// its head gets the rest (its tail) afterwards.
+constexpr uint32_t kHeadSamples = 256;  // sampled keys kept per tile
+struct HeadState {
+    // Cleared before each view, one block of zero_words: ctrl, sampled,
+    // tail_n, bits.
+    uint32_t* ctrl = nullptr;     // [8]: [0] tiles in `list`, [2..3] pairs placed in heads (u64)
+    uint32_t* sampled = nullptr;  // [8 * tiles]: sampled pairs, a counter per 32 bytes
+    uint32_t* tail_n = nullptr;   // [tiles]: tail pairs of a listed tile
+    uint32_t* bits = nullptr;     // [ceil(tiles / 32)]: listed tiles
+    size_t zero_words = 0;
+    uint32_t* keys = nullptr;        // [tiles][kHeadSamples]
+    uint32_t* limit = nullptr;       // [tiles]: last depth key of the head (0xffffffff: no tail)
+    uint32_t* tail_start = nullptr;  // [tiles]: first slot of a listed tile's tail
+    uint32_t* tail_at = nullptr;     // [tiles]: placement cursor of it
+    uint32_t* list = nullptr;        // [tiles]: tiles whose pixels want their tail
+    float* t = nullptr;              // [pixels]: transmittance after the head (tiles with a tail)
+};
+// Whether a view of `tiles` tiles over n splats takes depth-limited lists.
+bool heads_wanted(uint32_t n, uint32_t tiles);
+// limit[t] from every eighth splat's boxes and keys.
+cudaError_t launch_head_limits(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
+                               uint32_t tiles, const HeadState& h, cudaStream_t st);
+// launch_bin_count / launch_bin_place over the pairs of the heads; *total_all
+// += the pairs of the whole lists.
+cudaError_t launch_head_count(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
+                              uint32_t tiles, uint32_t chunks, uint32_t* hist, const HeadState& h,
+                              unsigned long long* total_all, cudaStream_t st);
+cudaError_t launch_head_place(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
+                              uint32_t tiles, uint32_t chunks, const uint32_t* hist, const uint32_t* tile_start,
+                              uint32_t capacity, uint2* pairs, uint32_t* err, const HeadState& h, cudaStream_t st);
+// The tails of the listed tiles, unsorted, after the heads in `pairs`; words[1]
+// as in launch_head_place, words[3] = listed tiles.
+cudaError_t launch_tail_place(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
+                              uint32_t tiles, uint32_t capacity, uint2* pairs, uint32_t* words, const HeadState& h,
+                              cudaStream_t st);
 // Segmented sort of the longest lists (sf_bin.cu): each list past min_list
 // entries (up to `lists` of them per frame) gets a key histogram of
 // kGiantBins buckets, cut into segments of about kGiantSegTarget entries that

@@ -470,7 +470,8 @@ struct TileShared {
 };
 
 // This CTA's part `sub` of one tile (block-uniform).
-template <int MODE, bool CULL, bool DETAIL, bool STATE, bool LAZY, uint32_t NT>
+// TAIL: the tile's tail, from the transmittances that its head left.
+template <int MODE, bool CULL, bool DETAIL, bool STATE, bool LAZY, bool TAIL, uint32_t NT>
 __device__ __forceinline__ void raster_tile(const RasterArgs& a, const uint32_t tile, const uint32_t sub) {
     extern __shared__ __align__(16) unsigned char s_tile[];
     TileShared<MODE, CULL, LAZY, NT>& sh = *reinterpret_cast<TileShared<MODE, CULL, LAZY, NT>*>(s_tile);
@@ -492,9 +493,10 @@ __device__ __forceinline__ void raster_tile(const RasterArgs& a, const uint32_t 
     uint32_t inside = 0;
     if (MODE == 3) inside = !a.mask || !in_bounds;  // pixels outside the image weigh nothing
     if ((MODE == 2 || (MODE == 3 && a.mask)) && in_bounds) inside = (a.mask[px / 32 + py * a.mask_wpr] >> (px % 32)) & 1u;
-    const uint32_t start = a.tile_start[tile], end = a.tile_start[tile + 1];
+    const uint32_t start = TAIL ? a.tail_start[tile] : a.tile_start[tile];
+    const uint32_t end = TAIL ? start + a.tail_n[tile] : a.tile_start[tile + 1];
     // A pixel takes entries while T >= 1/255; those outside the image start done.
-    PixelState ps{in_bounds ? 1.0f : 0.0f, 0.0f, 0.0f, 0.0f, 0u, 0u, 0u, 0u};
+    PixelState ps{!in_bounds ? 0.0f : TAIL ? a.head_t[(size_t)py * a.w + px] : 1.0f, 0.0f, 0.0f, 0.0f, 0u, 0u, 0u, 0u};
     if (ModeOf<MODE>::kWords) {
         for (uint32_t e = tid; e < kChunk; e += NT) {
             sm.acc0[0][e] = sm.acc0[1][e] = 0u;
@@ -532,7 +534,7 @@ __device__ __forceinline__ void raster_tile(const RasterArgs& a, const uint32_t 
             uint32_t pos = 0;
             // The first slab aims at kFirstSlab entries (most tiles saturate
             // well inside it), later ones at the full kSlab.
-            uint32_t target = kFirstSlab;
+            uint32_t target = TAIL ? kSlab : kFirstSlab;
             for (;;) {
                 // Pick [cur, sel] holding at most `target` of the values left
                 // (one whole bin of up to kSlab when the first bin alone is
@@ -616,6 +618,15 @@ __device__ __forceinline__ void raster_tile(const RasterArgs& a, const uint32_t 
             }
         }
     }
+    if (MODE != 0 && !TAIL && a.head_limit && a.head_limit[tile] != 0xffffffffu) {
+        // A head with a tail behind it: the transmittances are kept, and the
+        // tile is listed when one of this CTA's pixels takes more entries.
+        if (in_bounds) a.head_t[(size_t)py * a.w + px] = ps.T;
+        if (__syncthreads_or(ps.T >= 1.0f / 255.0f) && tid == 0) {
+            const uint32_t bit = 1u << (tile & 31u);
+            if (!(atomicOr(a.head_bits + (tile >> 5), bit) & bit)) a.head_list[atomicAdd(a.head_ctrl, 1u)] = tile;
+        }
+    }
     if (a.stats) {
         if (DETAIL) {
             const uint32_t e = __reduce_add_sync(0xffffffffu, ps.n_eval);
@@ -686,7 +697,17 @@ __global__ __launch_bounds__(NT) void raster_kernel(RasterArgs a) {
         // k < 0: the empty tiles (the counts sum to the tile count).
         tile = a.class_lists[(size_t)(k < 0 ? kSortClasses : k) * tiles + j];
     }
-    raster_tile<MODE, CULL, DETAIL, STATE, LAZY, NT>(a, tile, sub);
+    raster_tile<MODE, CULL, DETAIL, STATE, LAZY, false, NT>(a, tile, sub);
+}
+
+// The tails of the listed tiles, a CTA each in turn.
+template <int MODE>
+__global__ __launch_bounds__(256) void raster_tails_kernel(RasterArgs a) {
+    const uint32_t count = *a.head_ctrl;
+    for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
+        raster_tile<MODE, true, false, false, true, true, 256>(a, a.head_list[i], 0);
+        __syncthreads();
+    }
 }
 
 template <int MODE, bool CULL, bool DETAIL, bool STATE, bool LAZY, uint32_t NT>
@@ -716,6 +737,19 @@ cudaError_t raster_dispatch(const RasterArgs& a, uint32_t tiles, cudaStream_t st
     return raster_go<MODE, true, false, false, LAZY, 256>(a, tiles, st);
 }
 
+template <int MODE>
+cudaError_t tails_go(const RasterArgs& a, int sm_count, cudaStream_t st) {
+    constexpr size_t smem = sizeof(TileShared<MODE, true, true, 256>);
+    if (smem > 48 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(raster_tails_kernel<MODE>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+    }
+    const uint32_t tiles = a.tiles_x * a.tiles_y;
+    raster_tails_kernel<MODE><<<std::min(tiles, 3u * (uint32_t)std::max(sm_count, 1)), 256, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
 }  // namespace
 
 cudaError_t launch_raster(int mode, const RasterArgs& args, cudaStream_t stream) {
@@ -734,6 +768,23 @@ cudaError_t launch_raster(int mode, const RasterArgs& args, cudaStream_t stream)
         case 3:
             if (a.afg && a.abg && !lazy) e = raster_dispatch<3, false>(a, tiles, stream);
             break;
+        default: break;
+    }
+    if (e == cudaSuccess) note_launches(1);
+    return e;
+}
+
+cudaError_t launch_raster_tails(int mode, const RasterArgs& args, int sm_count, cudaStream_t stream) {
+    RasterArgs a = args;
+    a.lazy_min = 0;
+    a.stats = nullptr;
+    if (!a.pairs || !a.ext || !a.tail_start || !a.tail_n || !a.head_ctrl || !a.head_list || !a.head_t)
+        return cudaErrorInvalidValue;
+    cudaError_t e = cudaErrorInvalidValue;
+    switch (mode) {
+        case 1: e = tails_go<1>(a, sm_count, stream); break;
+        case 2: e = tails_go<2>(a, sm_count, stream); break;
+        case 3: e = tails_go<3>(a, sm_count, stream); break;
         default: break;
     }
     if (e == cudaSuccess) note_launches(1);

@@ -82,6 +82,7 @@ struct RoundLane {
     uint32_t* cnt = nullptr;
     uint32_t* lists = nullptr;
     GiantState giant;  // segmented sort of the longest lists
+    HeadState head;    // depth-limited lists
     SortStreams sort_streams;
 };
 
@@ -100,7 +101,7 @@ struct sf_round_t {
     std::vector<RoundLane> lanes;
     sf_view* views_dev = nullptr;
     sf_view* views_host = nullptr;  // pinned
-    uint32_t* words = nullptr;      // [views][16]: 0 visible, 1 err, 2 n32, 4..5 total u64, 6..14 binned stats
+    uint32_t* words = nullptr;      // [views][16]: 0 visible, 1 err, 2 n32, 3 tiles past their heads, 4..5 total u64, 6..14 binned stats
     uint32_t* words_host = nullptr; // pinned
     double* eig_dev = nullptr;
     double* eig_host = nullptr;     // pinned
@@ -131,6 +132,13 @@ struct sf_round_t {
     // graph includes the segmented sort of the longest lists for the view.
     std::vector<uint32_t> longest;
     std::vector<uint8_t> g_giant;
+    // Views whose heads left more than one in 128 of their tiles unsaturated
+    // (faint splats, a thin scene): they take whole lists until the splats
+    // change (8 views of 1M splats of opacity 0.05: 1.94 ms with whole lists,
+    // 2.22 ms with heads whose tails some tiles want). g_whole: as
+    // captured.
+    std::vector<uint8_t> whole, g_whole;
+    const void* whole_splats = nullptr;
     uint32_t chunks = 1;
     std::vector<const sf_mask_t*> g_masks;
 };
@@ -150,6 +158,8 @@ void lane_free(RoundLane& L) {
     dfree(L.giant.ctrl); dfree(L.giant.sel); dfree(L.giant.mm); dfree(L.giant.hist);
     dfree(L.giant.taken); dfree(L.giant.segs);
     L.giant.lists = L.giant.seg_cap = 0;
+    dfree(L.head.ctrl); dfree(L.head.keys); dfree(L.head.limit); dfree(L.head.t);
+    L.head = HeadState();
     sort_streams_destroy(&L.sort_streams);
     if (L.stream) cudaStreamDestroy(L.stream);
     if (L.join) cudaEventDestroy(L.join);
@@ -180,6 +190,28 @@ cudaError_t lane_alloc(sf_round_t* r, RoundLane& L, uint64_t cap) {
         RA(L.giant.hist, (size_t)L.giant.lists * kGiantBins);
         RA(L.giant.taken, r->max_tiles);
         RA(L.giant.segs, L.giant.seg_cap);
+    }
+    uint32_t head_tiles = 0;
+    uint64_t head_pixels = 0;
+    for (uint32_t v = 0; v < r->views; ++v) {
+        const uint32_t tiles = ((r->w[v] + 15) / 16) * ((r->h[v] + 15) / 16);
+        if (!heads_wanted(n, tiles)) continue;
+        head_tiles = std::max(head_tiles, tiles);
+        head_pixels = std::max<uint64_t>(head_pixels, (uint64_t)r->w[v] * r->h[v]);
+    }
+    if (head_tiles) {
+        HeadState& H = L.head;
+        H.zero_words = 8 + 9 * (size_t)head_tiles + (head_tiles + 31) / 32;
+        RA(H.ctrl, H.zero_words);
+        H.sampled = H.ctrl + 8;
+        H.tail_n = H.sampled + 8 * (size_t)head_tiles;
+        H.bits = H.tail_n + head_tiles;
+        RA(H.keys, (size_t)head_tiles * kHeadSamples);
+        RA(H.limit, 4 * (size_t)head_tiles);
+        H.tail_start = H.limit + head_tiles;
+        H.tail_at = H.tail_start + head_tiles;
+        H.list = H.tail_at + head_tiles;
+        RA(H.t, head_pixels);
     }
 #undef RA
     if ((e = cudaMalloc(&L.scan_tmp, scan_temp_bytes(std::max(n, r->max_tiles + 1)))) != cudaSuccess) return e;
@@ -245,10 +277,32 @@ cudaError_t depth_sorted_isects(sf_round_t* r, RoundLane& L, uint32_t n, uint32_
     return cudaSuccess;
 }
 
+// The raster's part in depth-limited lists: listing the tiles that want their
+// tails, then drawing those.
+void set_heads(const RoundLane& L, RasterArgs& a) {
+    a.head_limit = L.head.limit;
+    a.head_ctrl = L.head.ctrl;
+    a.head_bits = L.head.bits;
+    a.head_list = L.head.list;
+    a.head_t = L.head.t;
+    a.tail_start = L.head.tail_start;
+    a.tail_n = L.head.tail_n;
+}
+cudaError_t enqueue_tails(sf_round_t* r, RoundLane& L, uint32_t v, int mode, const RasterArgs& heads,
+                          cudaStream_t st) {
+    uint2* pairs = reinterpret_cast<uint2*>(L.tid_a);
+    cudaError_t e = launch_tail_place(L.bbox, L.keys, r->n, heads.tiles_x, heads.tiles_x * heads.tiles_y,
+                                      (uint32_t)L.cap, pairs, r->words + 16 * v, L.head, st);
+    if (e != cudaSuccess) return e;
+    RasterArgs a = heads;
+    a.pairs = pairs;
+    return launch_raster_tails(mode, a, r->sm_count, st);
+}
+
 // Responsibility (or evidence) raster of view v and its EIG.
 cudaError_t raster_and_eig(sf_round_t* r, RoundLane& L, uint32_t v, uint32_t tx, uint32_t ty, const uint32_t* gids,
                            const uint2* pairs, const float* beta_a, const float* beta_b, const float* lut, int mode,
-                           cudaStream_t st) {
+                           bool heads, cudaStream_t st) {
     cudaError_t e;
     const uint32_t n = r->n;
     const uint32_t w = r->w[v], h = r->h[v];
@@ -270,6 +324,7 @@ cudaError_t raster_and_eig(sf_round_t* r, RoundLane& L, uint32_t v, uint32_t tx,
     a.ext = L.ext;
     a.split = r->tuning.raster_split;
     a.scale = (float)((uint64_t)1 << frac_bits(w, h));
+    if (heads) set_heads(L, a);
     if (bg) {
         // Evidence: the mask splits each pixel's weights into fg / bg.
         a.mask = r->masks[v]->bits;
@@ -281,6 +336,7 @@ cudaError_t raster_and_eig(sf_round_t* r, RoundLane& L, uint32_t v, uint32_t tx,
         a.resp = resp;
         if ((e = launch_raster(1, a, st)) != cudaSuccess) return e;
     }
+    if (heads && (e = enqueue_tails(r, L, v, bg ? 2 : 1, a, st)) != cudaSuccess) return e;
     if (beta_a) {
         // Under masks the EIG sees eps = fg + bg, the same words mode 1 sums.
         if ((e = launch_eig(mode, beta_a, beta_b, resp, n, a.scale, lut, L.partials, r->eig_blocks,
@@ -294,7 +350,7 @@ cudaError_t raster_and_eig(sf_round_t* r, RoundLane& L, uint32_t v, uint32_t tx,
 // and, with a posterior, the EIG over fg + bg.
 cudaError_t adjoint_and_eig(sf_round_t* r, RoundLane& L, uint32_t v, uint32_t tx, uint32_t ty,
                             const uint32_t* gids, const float* beta_a, const float* beta_b, const float* lut,
-                            int mode, cudaStream_t st) {
+                            int mode, bool heads, cudaStream_t st) {
     cudaError_t e;
     const uint32_t n = r->n;
     const uint32_t w = r->w[v], h = r->h[v];
@@ -318,7 +374,9 @@ cudaError_t adjoint_and_eig(sf_round_t* r, RoundLane& L, uint32_t v, uint32_t tx
     a.abg = bg;
     if ((e = cudaMemsetAsync(fg, 0, (size_t)n * 4, st)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(bg, 0, (size_t)n * 4, st)) != cudaSuccess) return e;
+    if (heads) set_heads(L, a);
     if ((e = launch_raster(3, a, st)) != cudaSuccess) return e;
+    if (heads && (e = enqueue_tails(r, L, v, 3, a, st)) != cudaSuccess) return e;
     if (beta_a)
         return launch_eig_real(mode, beta_a, beta_b, fg, bg, n, lut, L.partials, r->eig_blocks, r->eig_dev + v, st,
                                r->h0);
@@ -342,7 +400,31 @@ cudaError_t enqueue_view(sf_round_t* r, RoundLane& L, uint32_t v, const sf_splat
     if ((e = launch_project(dummy, sp.attr, sp.geom, sp.sh, n, sp.K, po, st, r->views_dev + v)) != cudaSuccess) return e;
     const uint32_t *tids = nullptr, *gids = nullptr;
     const uint2* lazy_pairs = nullptr;
-    if (r->tuning.isect_build == SF_ISECTS_BINNED && L.hist) {
+    const bool heads = r->tuning.isect_build == SF_ISECTS_BINNED && L.hist && L.head.ctrl &&
+                       (r->adjoint || r->tuning.raster_order == SF_ORDER_SORTED) && !r->whole[v] &&
+                       heads_wanted(n, tiles);
+    if (heads) {
+        // Only the nearest pairs of each tile are counted, placed and sorted;
+        // words[4..5] gets the pairs of the whole lists.
+        const HeadState& H = L.head;
+        unsigned long long* placed = reinterpret_cast<unsigned long long*>(H.ctrl + 2);
+        uint2* pairs = reinterpret_cast<uint2*>(L.tid_a);
+        if ((e = cudaMemsetAsync(H.ctrl, 0, 4 * H.zero_words, st)) != cudaSuccess) return e;
+        if ((e = launch_head_limits(L.bbox, L.keys, n, tx, tiles, H, st)) != cudaSuccess) return e;
+        if ((e = launch_head_count(L.bbox, L.keys, n, tx, tiles, r->chunks, L.hist, H, total, st)) != cudaSuccess)
+            return e;
+        if ((e = launch_bin_colscan(L.hist, r->chunks, tiles, L.cnt, L.lists, words, st)) != cudaSuccess) return e;
+        if ((e = launch_tile_scan(L.cnt, tiles + 1, (uint32_t)L.cap, L.tile_start, placed, st)) != cudaSuccess) return e;
+        if ((e = launch_head_place(L.bbox, L.keys, n, tx, tiles, r->chunks, L.hist, L.tile_start, (uint32_t)L.cap,
+                                   pairs, words + 1, H, st)) != cudaSuccess)
+            return e;
+        uint32_t grids[kSortClasses];
+        tile_sort_bounds(n, tiles, grids);
+        if ((e = launch_tile_sorts(grids, L.lists, words, tiles, L.tile_start, (uint32_t)L.cap, pairs, L.gid_e,
+                                   nullptr, L.tid_e, r->sm_count, st, &L.sort_streams, nullptr)) != cudaSuccess)
+            return e;
+        gids = L.gid_e;
+    } else if (r->tuning.isect_build == SF_ISECTS_BINNED && L.hist) {
         // Binned build with device-side counts: the sorts take every tile as
         // the bound of each class and read the class sizes on the device.
         if ((e = launch_bin_count(L.bbox, n, tx, tiles, r->chunks, L.hist, st)) != cudaSuccess) return e;
@@ -370,8 +452,8 @@ cudaError_t enqueue_view(sf_round_t* r, RoundLane& L, uint32_t v, const sf_splat
         if ((e = depth_sorted_isects(r, L, n, tx, tiles, words, total, st, &tids, &gids)) != cudaSuccess)
             return e;
     }
-    if (r->adjoint) return adjoint_and_eig(r, L, v, tx, ty, gids, beta_a, beta_b, lut, mode, st);
-    return raster_and_eig(r, L, v, tx, ty, gids, lazy_pairs, beta_a, beta_b, lut, mode, st);
+    if (r->adjoint) return adjoint_and_eig(r, L, v, tx, ty, gids, beta_a, beta_b, lut, mode, heads, st);
+    return raster_and_eig(r, L, v, tx, ty, gids, lazy_pairs, beta_a, beta_b, lut, mode, heads, st);
 }
 
 }  // namespace
@@ -446,6 +528,7 @@ int build_graph(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, int
     r->g_radix = r->tuning.radix_bits;
     r->g_masks = r->masks;
     for (uint32_t v = 0; v < r->views; ++v) r->g_giant[v] = giant_wanted(r->longest[v], r->g_giant[v]);
+    r->g_whole = r->whole;
     return SF_OK;
 }
 
@@ -460,6 +543,10 @@ bool giant_changed(const sf_round_t* r) {
 int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const sf_camera* cams, int mode,
               cudaStream_t user) {
     for (uint32_t v = 0; v < r->views; ++v) view_for_camera(cams[v], r->w[v], r->h[v], &r->views_host[v]);
+    if (r->whole_splats != sp) {
+        r->whole.assign(r->views, 0);
+        r->whole_splats = sp;
+    }
     for (int attempt = 0; attempt < 4; ++attempt) {
         const uint32_t lanes = std::max(1u, std::min(r->tuning.lanes ? r->tuning.lanes : 4u, r->views));
         if (r->lanes.size() != lanes || r->lanes[0].cap < r->want_cap) {
@@ -469,7 +556,7 @@ int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const
             r->g_adjoint != (int)r->adjoint ||
             r->g_build != r->tuning.isect_build ||
             r->g_order != r->tuning.raster_order || r->g_split != r->tuning.raster_split ||
-            r->g_radix != r->tuning.radix_bits || r->g_masks != r->masks ||
+            r->g_radix != r->tuning.radix_bits || r->g_masks != r->masks || r->g_whole != r->whole ||
             giant_changed(r)) {
             const int rc = build_graph(r, sp, beta, mode);
             if (rc != SF_OK) return rc;
@@ -494,7 +581,11 @@ int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const
             r->longest[v] = w[6];
             if (w[1] & SF_DEV_ERR_CAPACITY) over = true;
         }
-        if (!over) return SF_OK;
+        if (!over) {
+            for (uint32_t v = 0; v < r->views; ++v)
+                if (r->words_host[16 * v + 3] > ((r->w[v] + 15) / 16) * ((r->h[v] + 15) / 16) / 128) r->whole[v] = 1;
+            return SF_OK;
+        }
         if (worst > (1ull << 30) - 1) return rfail(SF_ERR_CAPACITY, "intersection count exceeds 2^30-1");
         r->want_cap = next_pow2(worst);
         std::fprintf(stderr, "splatfield_b200: round capacity grown to %llu intersections per view\n",
