@@ -301,7 +301,7 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t x, uint32_t* s32, uint32
 // A tile's pixels are saturated after its first few hundred entries: the
 // raster of a 512x512 view of 1M splats walks 5 to 8% of its pairs, but all of
 // them are placed and sorted. So a round's view places heads only:
-//   1. head_sample: the depth keys of every eighth splat, per tile;
+//   1. head_sample: the depth keys of every 32nd splat, per tile;
 //   2. head_pick: per tile the key below which about kHeadTarget of its pairs
 //      lie (tiles whose whole list is about that short get no limit);
 //   3. count, place, sorts and raster over the pairs up to the limit. A tile

@@ -239,7 +239,7 @@ struct HeadState {
 };
 // Whether a view of `tiles` tiles over n splats takes depth-limited lists.
 bool heads_wanted(uint32_t n, uint32_t tiles);
-// limit[t] from every eighth splat's boxes and keys.
+// limit[t] from every 32nd splat's boxes and keys.
 cudaError_t launch_head_limits(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
                                uint32_t tiles, const HeadState& h, cudaStream_t st);
 // launch_bin_count / launch_bin_place over the pairs of the heads; *total_all
