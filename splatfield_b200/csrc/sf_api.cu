@@ -145,6 +145,8 @@ struct sf_scratch_t {
         cudaGraphExec_t exec = nullptr;
         uint32_t kernels = 0;           // kernel nodes of exec
         cudaStream_t stream = nullptr;  // capture stream
+        cudaStream_t status = nullptr;  // capture stream of the status words' copy
+        cudaEvent_t status_fork = nullptr, status_join = nullptr;
         sf_view* view_dev = nullptr;
         sf_view* view_host = nullptr;   // pinned
         const void* splats = nullptr;
@@ -572,6 +574,9 @@ int frame_graph_capture(sf_splats sp, sf_scratch s) {
         g.exec = nullptr;
     }
     if (!g.stream) SF_CK(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
+    if (!g.status) SF_CK(cudaStreamCreateWithFlags(&g.status, cudaStreamNonBlocking));
+    if (!g.status_fork) SF_CK(cudaEventCreateWithFlags(&g.status_fork, cudaEventDisableTiming));
+    if (!g.status_join) SF_CK(cudaEventCreateWithFlags(&g.status_join, cudaEventDisableTiming));
     if (!g.view_dev) SF_CK(dalloc(&g.view_dev, 1));
     if (!g.ring) SF_CK(dalloc(&g.ring, 16 * (size_t)kFrameRing));
     if (!g.view_host) SF_CK(cudaMallocHost(reinterpret_cast<void**>(&g.view_host), sizeof(sf_view)));
@@ -601,6 +606,12 @@ int frame_graph_capture(sf_splats sp, sf_scratch s) {
     if (e == cudaSuccess)
         e = launch_bin_place(s->bbox, s->depth_keys, n, s->tiles_x, tiles, s->bin_chunks, s->bin_hist,
                              s->tile_start, cap, pairs, words + 1, st);
+    // No kernel after the placement writes the status words, so they are
+    // copied to the host beside the sorts and the raster.
+    if (e == cudaSuccess) e = cudaEventRecord(g.status_fork, st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(g.status, g.status_fork, 0);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(s->host_words, words, 64, cudaMemcpyDeviceToHost, g.status);
+    if (e == cudaSuccess) e = cudaEventRecord(g.status_join, g.status);
     if (e == cudaSuccess && order != SF_ORDER_IN_RASTER) {
         uint32_t grids[kSortClasses];
         tile_sort_bounds(n, tiles, grids);
@@ -632,6 +643,7 @@ int frame_graph_capture(sf_splats sp, sf_scratch s) {
         }
         e = launch_raster(0, a, st);
     }
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, g.status_join, 0);
     cudaGraph_t graph = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(st, &graph);
     g.kernels = (uint32_t)(launches() - launches0);
@@ -702,7 +714,6 @@ int frame_graph_render(sf_splats sp, sf_scratch s, const sf_camera* cam, uint32_
         SF_CK(cudaMemcpyAsync(g.view_dev, g.view_host, sizeof(sf_view), cudaMemcpyHostToDevice, st));
         SF_CK(cudaGraphLaunch(g.exec, st));
         note_launches(g.kernels);
-        SF_CK(cudaMemcpyAsync(s->host_words, s->words, 64, cudaMemcpyDeviceToHost, st));
         if (host_out)
             SF_CK(cudaMemcpy2DAsync(host_out, (size_t)w * 4, s->bitmap, (size_t)s->row_stride * 4, (size_t)w * 4,
                                     h, cudaMemcpyDeviceToHost, st));
@@ -1134,6 +1145,9 @@ int sf_scratch_destroy(sf_scratch s) {
     sort_streams_destroy(&s->sort_streams);
     if (s->fg.exec) cudaGraphExecDestroy(s->fg.exec);
     if (s->fg.stream) cudaStreamDestroy(s->fg.stream);
+    if (s->fg.status) cudaStreamDestroy(s->fg.status);
+    if (s->fg.status_fork) cudaEventDestroy(s->fg.status_fork);
+    if (s->fg.status_join) cudaEventDestroy(s->fg.status_join);
     dfree(s->fg.view_dev);
     if (s->fg.view_host) cudaFreeHost(s->fg.view_host);
     if (s->fg.copy) {
