@@ -351,8 +351,20 @@ int prepare_binned(sf_scratch s, uint32_t n, uint32_t tiles, cudaStream_t st, bo
     SF_CK(launch_bin_colscan(s->bin_hist, s->bin_chunks, tiles, s->bin_cnt, s->bin_lists, words, st));
     // The capacity follows the total below: the starts are not cut.
     SF_CK(launch_tile_scan(s->bin_cnt, tiles + 1, 0xffffffffu, s->tile_start, total_dev, st));
-    SF_CK(cudaMemcpyAsync(s->host_words, words, 64, cudaMemcpyDeviceToHost, st));
-    SF_CK(cudaStreamSynchronize(st));
+    // The words are read on a side stream while the placement runs against the
+    // present capacity (it drops what lies past it), so the GPU is not idle
+    // while the host waits for them.
+    if (!s->sort_streams.s[0]) SF_CK(sort_streams_create(&s->sort_streams));
+    cudaStream_t side = s->sort_streams.s[0];
+    SF_CK(cudaEventRecord(s->sort_streams.e[0], st));
+    SF_CK(cudaStreamWaitEvent(side, s->sort_streams.e[0], 0));
+    SF_CK(cudaMemcpyAsync(s->host_words, words, 64, cudaMemcpyDeviceToHost, side));
+    const auto place = [&] {
+        return launch_bin_place(s->bbox, s->depth_keys, n, s->tiles_x, tiles, s->bin_chunks, s->bin_hist,
+                                s->tile_start, (uint32_t)s->cap, reinterpret_cast<uint2*>(s->tid_a), words + 1, st);
+    };
+    SF_CK(place());
+    SF_CK(cudaStreamSynchronize(side));
     const uint32_t* hw = s->host_words;
     if (hw[1] & SF_DEV_ERR_TIMEOUT) return fail(SF_ERR_TIMEOUT, "device look-back wait timed out");
     uint64_t total = 0;
@@ -364,11 +376,12 @@ int prepare_binned(sf_scratch s, uint32_t n, uint32_t tiles, cudaStream_t st, bo
     if (total > s->cap) {
         std::fprintf(stderr, "splatfield_b200: intersection capacity %llu reached (%llu needed); growing\n",
                      (unsigned long long)s->cap, (unsigned long long)total);
+        SF_CK(cudaStreamSynchronize(st));
         SF_CK(grow_isects(s, total));
+        SF_CK(cudaMemsetAsync(words + 1, 0, 4, st));
+        SF_CK(place());
     }
     uint2* pairs = reinterpret_cast<uint2*>(s->tid_a);
-    SF_CK(launch_bin_place(s->bbox, s->depth_keys, n, s->tiles_x, tiles, s->bin_chunks, s->bin_hist,
-                           s->tile_start, (uint32_t)s->cap, pairs, words + 1, st));
     s->lazy = order != SF_ORDER_SORTED;
     s->lazy_min = order == SF_ORDER_HYBRID ? kBinSharedMax : 0u;
     if (order == SF_ORDER_IN_RASTER) {
@@ -381,7 +394,6 @@ int prepare_binned(sf_scratch s, uint32_t n, uint32_t tiles, cudaStream_t st, bo
         // some list is long enough to gain from it.
         GiantState giant = s->giant;
         giant.min_list = kGiantMinAlone;
-        if (!s->sort_streams.s[0]) SF_CK(sort_streams_create(&s->sort_streams));
         SF_CK(launch_tile_sorts(grids, s->bin_lists, words, tiles, s->tile_start, (uint32_t)s->cap, pairs,
                                 s->gid_e, want_tile_ids ? s->tid_e : nullptr, s->tid_e, s->ctx->sm_count, st,
                                 &s->sort_streams, hw[6] > kGiantMinAlone ? &giant : nullptr));

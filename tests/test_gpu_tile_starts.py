@@ -43,3 +43,24 @@ def test_frame_past_the_capacity_is_drawn_again_whole(ctx, oracle_mod):
     got = splats.render_frames_to_host(scratch, [cam] * 5, (w, h))
     for img in got:
         np.testing.assert_array_equal(img, want["bitmap"][:, :w])
+
+
+def test_prepare_past_the_capacity_places_again(ctx, oracle_mod):
+    """The placement runs before the host knows the total: lists that outgrow
+    the capacity of an earlier frame are placed again after the growth."""
+    n, w, h = 6000, 640, 480
+    attr, sh = synth.scene_uniform(n, 1, 5)
+    big = attr.reshape(11, n).copy()
+    big[7:10] += 4.0
+    pos, tgt = (0.1, 0.0, -2.5), (0.0, 0.0, 0.0)
+    cam = sf.look_at(pos, tgt)
+    small, splats = sf.Splats(attr, sh), sf.Splats(big.reshape(-1), sh)
+    want = oracle_mod.prepare(oracle_mod.look_at(pos, tgt), w, h, big.reshape(-1), sh, 1)
+    scratch = sf.RenderScratch(n, (w, h))
+    small.prepare_isects(scratch, cam, (w, h))
+    before = scratch.capacity()
+    assert want["gaussian_ids"].size > before
+    ti = splats.prepare_isects(scratch, cam, (w, h))
+    assert scratch.capacity() > before
+    np.testing.assert_array_equal(ti.gaussian_ids().read(), want["gaussian_ids"])
+    np.testing.assert_array_equal(ti.tile_ids().read(), want["tile_ids"])
