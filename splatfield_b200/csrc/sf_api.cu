@@ -331,6 +331,9 @@ cudaError_t scratch_build(sf_scratch s, uint32_t total, uint32_t w, uint32_t h) 
         if ((e = dalloc(&s->words, kStatusWords)) != cudaSuccess) return e;
         s->stats = reinterpret_cast<unsigned long long*>(s->words + 16);
         if ((e = cudaMallocHost(reinterpret_cast<void**>(&s->host_words), 64)) != cudaSuccess) return e;
+        // Streams of the frame's side branches, here and not in the first
+        // frame (80 us of it).
+        if ((e = sort_streams_create(&s->sort_streams)) != cudaSuccess) return e;
     }
     // Capacity: keep the larger of the growth hint and the reference's first
     // frame rule min(tiles*total, 2^22) (render.rs:146-147, 177-183).
@@ -354,7 +357,6 @@ int prepare_binned(sf_scratch s, uint32_t n, uint32_t tiles, cudaStream_t st, bo
     // The words are read on a side stream while the placement runs against the
     // present capacity (it drops what lies past it), so the GPU is not idle
     // while the host waits for them.
-    if (!s->sort_streams.s[0]) SF_CK(sort_streams_create(&s->sort_streams));
     cudaStream_t side = s->sort_streams.s[0];
     SF_CK(cudaEventRecord(s->sort_streams.e[0], st));
     SF_CK(cudaStreamWaitEvent(side, s->sort_streams.e[0], 0));
@@ -592,7 +594,6 @@ int frame_graph_capture(sf_splats sp, sf_scratch s) {
     if (!g.view_dev) SF_CK(dalloc(&g.view_dev, 1));
     if (!g.ring) SF_CK(dalloc(&g.ring, 16 * (size_t)kFrameRing));
     if (!g.view_host) SF_CK(cudaMallocHost(reinterpret_cast<void**>(&g.view_host), sizeof(sf_view)));
-    if (!s->sort_streams.s[0]) SF_CK(sort_streams_create(&s->sort_streams));
     const uint32_t n = sp->n;
     const uint32_t tiles = s->tiles_x * s->tiles_y;
     const uint32_t cap = (uint32_t)s->cap;
@@ -1132,6 +1133,7 @@ int sf_scratch_create(sf_ctx ctx, uint32_t total, uint32_t w, uint32_t h, sf_scr
         if (e != cudaSuccess) {
             scratch_free_frame(s);
             scratch_free_isects(s);
+            sort_streams_destroy(&s->sort_streams);
             delete s;
             return fail(e == cudaErrorMemoryAllocation ? SF_ERR_NOMEM : SF_ERR_CUDA, cudaGetErrorString(e));
         }
