@@ -1,6 +1,7 @@
 // Handle types shared by the C ABI translation units (sf_api.cu, sf_round.cu).
 #pragma once
 #include <cstdint>
+#include <mutex>
 #include <string>
 #include "sf_internal.h"
 
@@ -8,6 +9,12 @@ struct sf_ctx_t {
     int device = 0;
     int sm_count = 148;
     float* lut = nullptr;  // f32 entropy LUT, built on first use
+    // Page-locked error words of the sort and scan scratches: one page, taken
+    // by the first of them and held until the context goes (page-locking costs
+    // a millisecond or more, a whole scratch 0.4). word_used: a bit per slot.
+    std::mutex word_mu;
+    uint32_t* word_page = nullptr;
+    uint64_t word_used = 0;
 };
 
 struct sf_splats_t {
@@ -38,8 +45,7 @@ struct sf_beta_t {
     float *a = nullptr, *b = nullptr;
     double* partials = nullptr;
     uint32_t blocks = 1;
-    double* out = nullptr;
-    double* host_out = nullptr;
+    double* host_out = nullptr;  // pinned; the last kernel of a synchronous EIG writes it
     // Localization scratch (allocated on first use): [blocks][4] partials,
     // [8] results, pinned mirror of the results.
     double* loc_partials = nullptr;
