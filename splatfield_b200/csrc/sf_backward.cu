@@ -162,6 +162,9 @@ __global__ __launch_bounds__(kBwdThreads, 4) void raster_bwd_kernel(BwdArgs a) {
     };
     const f32x2 nfx = both(-fx), nfy = both(-fy);
     PairRec<true>* const recs = sm.pairs[warp];
+    // A pixel of the warp has a dL/dcolour that is not finite (or near the
+    // largest float): its zeros are then selected, not multiplied.
+    const bool wild = __any_sync(0xffffffffu, !((fabsf(g.x) + fabsf(g.y)) + fabsf(g.z) < INFINITY));
     // 1 / (1 - alpha), alpha in [0, 0.999]: the approximate reciprocal and one
     // Newton-Raphson step (within an ulp of the rounded quotient).
     auto inv_through = [](float alpha) {
@@ -219,8 +222,17 @@ __global__ __launch_bounds__(kBwdThreads, 4) void raster_bwd_kernel(BwdArgs a) {
         const f32x2 w2 = pack2(wa, wb), d2 = pack2(da, db);
         const f32x2 dp = mul2(d2, pack2(-ala, -alb));
         const f32x2 mx = mul2(dp, dx), my = mul2(dp, dy);
-        const f32x2 v[9] = {mx, my, mul2(mx, dx), mul2(mx, dy), mul2(my, dy), mul2(both(g.x), w2),
-                            mul2(both(g.y), w2), mul2(both(g.z), w2), mul2(d2, pack2(oka ? ea : 0.0f, okb ? eb : 0.0f))};
+        f32x2 v[9] = {mx, my, mul2(mx, dx), mul2(mx, dy), mul2(my, dy), mul2(both(g.x), w2),
+                      mul2(both(g.y), w2), mul2(both(g.z), w2), mul2(d2, pack2(oka ? ea : 0.0f, okb ? eb : 0.0f))};
+        if (wild) {
+            // w = 0 does not clear an infinite or NaN dL/dcolour.
+#pragma unroll
+            for (uint32_t q = 5; q < 8; ++q) {
+                float va, vb;
+                unpack2(v[q], va, vb);
+                v[q] = pack2(oka ? va : 0.0f, okb ? vb : 0.0f);
+            }
+        }
         float x[16], y[2];
 #pragma unroll
         for (uint32_t q = 0; q < 8; ++q) unpack2(v[q], x[q], x[8 + q]);
