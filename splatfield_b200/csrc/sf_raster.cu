@@ -298,7 +298,8 @@ __device__ bool composite_list(const RasterArgs& a, Stage<MODE, CULL, NT>& sm, I
     };
     // Up to 32 candidates [g32, g32 + 32) of buffer b, of which this lane's is
     // walked when `hit`: the hits are packed two by two into recs in list
-    // order (an odd last one beside an entry of opacity 0) and composited.
+    // order (an odd last one beside an entry that no pixel takes) and
+    // composited.
     auto walk = [&](uint32_t b, uint32_t g32, bool hit, const float4& g0, const float4& g1, uint32_t pos0) {
         const uint32_t word = __ballot_sync(0xffffffffu, hit);
         const uint32_t hits = (uint32_t)__popc(word);
@@ -325,7 +326,8 @@ __device__ bool composite_list(const RasterArgs& a, Stage<MODE, CULL, NT>& sm, I
         }
         if ((hits & 1u) && lane == 0) {
             auto& r = recs[hits >> 1];
-            r.x[1] = r.y[1] = r.nhx[1] = r.ncy[1] = r.nhz[1] = r.op[1] = r.npm[1] = 0.0f;
+            r.x[1] = r.y[1] = r.nhx[1] = r.ncy[1] = r.nhz[1] = r.op[1] = 0.0f;
+            r.npm[1] = INFINITY;  // past every power: not an evaluated pair either
             if (kColor) r.r[1] = r.g[1] = r.b[1] = 0.0f;
             r.j[1] = g32;
         }
