@@ -1411,10 +1411,15 @@ cudaError_t launch_sort_kernel(K kernel, uint32_t threads, size_t smem, uint32_t
     return cudaGetLastError();
 }
 
-cudaError_t smem_opt_in(const void* fn, size_t smem) {
+// A launch of `smem` bytes, of at most `most` in any launch of the kernel. The
+// limit is one per kernel and device, so it is only ever set to `most`: set to
+// each launch's own size, it would be lowered under another thread's launch.
+cudaError_t smem_opt_in(const void* fn, size_t smem, size_t most) {
     if (smem <= 40 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
 }
+constexpr size_t kBinSmem = 4 * (size_t)kBinMaxTiles, kHeadSmem = 8 * (size_t)kHeadMaxTiles,
+                 kTailSmem = 4 * (size_t)kHeadMaxTiles;
 
 }  // namespace
 
@@ -1452,7 +1457,7 @@ void tile_sort_bounds(uint32_t n, uint32_t tiles, uint32_t grids[kSortClasses]) 
 cudaError_t launch_bin_count(const uint2* bbox, uint32_t n, uint32_t tiles_x, uint32_t tiles, uint32_t chunks,
                              uint32_t* hist, cudaStream_t st) {
     const size_t smem = (size_t)tiles * 4;
-    cudaError_t e = smem_opt_in((const void*)bin_count_kernel, smem);
+    cudaError_t e = smem_opt_in((const void*)bin_count_kernel, smem, kBinSmem);
     if (e != cudaSuccess) return e;
     e = launch_pdl(bin_count_kernel, chunks, kBinThreads, smem, st, bbox, n, bin_chunk_size(n, chunks), tiles_x,
                    tiles, hist);
@@ -1473,7 +1478,7 @@ cudaError_t launch_bin_place(const uint2* bbox, const uint32_t* depth_keys, uint
                              uint32_t tiles, uint32_t chunks, const uint32_t* hist, const uint32_t* tile_start,
                              uint32_t capacity, uint2* pairs, uint32_t* err, cudaStream_t st) {
     const size_t smem = (size_t)tiles * 4;
-    cudaError_t e = smem_opt_in((const void*)bin_place_kernel, smem);
+    cudaError_t e = smem_opt_in((const void*)bin_place_kernel, smem, kBinSmem);
     if (e != cudaSuccess) return e;
     e = launch_pdl(bin_place_kernel, chunks, kBinThreads, smem, st, bbox, depth_keys, n, bin_chunk_size(n, chunks),
                    tiles_x, tiles, hist, tile_start, capacity, pairs, err);
@@ -1498,7 +1503,7 @@ cudaError_t launch_head_count(const uint2* bbox, const uint32_t* depth_keys, uin
                               uint32_t tiles, uint32_t chunks, uint32_t* hist, const HeadState& h,
                               unsigned long long* total_all, cudaStream_t st) {
     const size_t smem = (size_t)tiles * 8;
-    const cudaError_t e = smem_opt_in((const void*)head_count_kernel, smem);
+    const cudaError_t e = smem_opt_in((const void*)head_count_kernel, smem, kHeadSmem);
     if (e != cudaSuccess) return e;
     head_count_kernel<<<chunks, kBinThreads, smem, st>>>(bbox, depth_keys, n, bin_chunk_size(n, chunks), tiles_x, tiles,
                                                          hist, h.limit, total_all);
@@ -1510,7 +1515,7 @@ cudaError_t launch_head_place(const uint2* bbox, const uint32_t* depth_keys, uin
                               uint32_t tiles, uint32_t chunks, const uint32_t* hist, const uint32_t* tile_start,
                               uint32_t capacity, uint2* pairs, uint32_t* err, const HeadState& h, cudaStream_t st) {
     const size_t smem = (size_t)tiles * 8;
-    cudaError_t e = smem_opt_in((const void*)head_place_kernel, smem);
+    cudaError_t e = smem_opt_in((const void*)head_place_kernel, smem, kHeadSmem);
     if (e != cudaSuccess) return e;
     e = launch_pdl(head_place_kernel, chunks, kBinThreads, smem, st, bbox, depth_keys, n, bin_chunk_size(n, chunks),
                    tiles_x, tiles, hist, tile_start, capacity, pairs, err, (const uint32_t*)h.limit);
@@ -1523,8 +1528,8 @@ cudaError_t launch_tail_place(const uint2* bbox, const uint32_t* depth_keys, uin
                               cudaStream_t st) {
     const uint32_t blocks = std::min((n + kTailThreads - 1) / kTailThreads, 296u);
     const size_t smem = (size_t)tiles * 4;
-    cudaError_t e = smem_opt_in((const void*)tail_count_kernel, smem);
-    if (e == cudaSuccess) e = smem_opt_in((const void*)tail_place_kernel, smem);
+    cudaError_t e = smem_opt_in((const void*)tail_count_kernel, smem, kTailSmem);
+    if (e == cudaSuccess) e = smem_opt_in((const void*)tail_place_kernel, smem, kTailSmem);
     if (e != cudaSuccess) return e;
     tail_count_kernel<<<blocks, kTailThreads, smem, st>>>(bbox, depth_keys, n, tiles_x, tiles, h);
     tail_plan_kernel<<<1, 1024, 0, st>>>(h, capacity, words + 3);

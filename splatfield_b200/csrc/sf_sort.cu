@@ -606,9 +606,11 @@ cudaError_t radix_sort_bits(const uint32_t* keys_in, const uint32_t* vals_in, ui
     if (e != cudaSuccess) return e;
     if (parts == 0) { *out_in_b = 0; return cudaSuccess; }
     if (grid_n >= kWideHistN) {
+        // The limit is one per kernel and device: always set for the most
+        // passes, so that no call lowers it under another thread's launch.
         const size_t smem = (size_t)passes * R * 32 * 4;
         e = cudaFuncSetAttribute(radix_histogram_wide_kernel<BITS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
+                                 kHistWords * 32 * 4);
         if (e != cudaSuccess) return e;
         radix_histogram_wide_kernel<BITS><<<(uint32_t)std::max(sm_count, 1), kWideHistThreads, smem, stream>>>(
             keys_in, n_dev, n, passes, bits, hist);
