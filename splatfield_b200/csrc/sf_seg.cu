@@ -199,9 +199,12 @@ __device__ __forceinline__ double entropy_delta(uint32_t i, const Eps& eps, cons
 // them for a few live lanes. Each warp instead queues the splats that have
 // weight, in index order, and evaluates 32 at a time. The partition and the
 // order of the sums depend on n alone, so a view's EIG is the same in a round
-// and by itself. FP64, 3M splats of which a 384x384 view weighs about a tenth:
-// 94 -> 34 us (at 5, 3 and 2 blocks per SM 37, 38 and 40 us); 60k splats 31 ->
-// 24 us.
+// and by itself. Whole calls against a thread per splat, with all, half and 7%
+// of the splats weighted: FP64 over 10M 1139 -> 1141, 1145 -> 638 and 1016 ->
+// 144 us, over 1M 134 -> 126, 135 -> 94 and 129 -> 45 us (blocks per SM 5, 4, 3
+// and 2 on the half of 10M: 660, 638, 668 and 707); LUT over 10M 204 -> 212,
+// 166 -> 142 and 154 -> 55 us, over 1M 46 -> 40, 40 -> 33 and 37 -> 23 us
+// (loads of two groups: 242, 222 at 90% and 69 us on the 10M).
 constexpr uint32_t kEigLoads = 4;  // groups of 32 splats whose weights a warp loads together
 template <int MODE, typename Eps>
 __global__ __launch_bounds__(kEigThreads, MODE == SF_EIG_FP64 ? 4 : 5) void eig_kernel(const float* __restrict__ a,
@@ -210,38 +213,60 @@ __global__ __launch_bounds__(kEigThreads, MODE == SF_EIG_FP64 ? 4 : 5) void eig_
                                                              double* __restrict__ partials,
                                                              const void* __restrict__ h0) {
     __shared__ double s_warp[kEigThreads / 32];
-    __shared__ uint32_t s_queue[kEigThreads / 32][64];
+    __shared__ uint32_t s_queue[kEigThreads / 32][32 * (kEigLoads + 1)];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lt = (1u << lane) - 1u;
     uint32_t* queue = s_queue[warp];
     uint32_t queued = 0;
     double acc = 0.0;
     const uint64_t stride = (uint64_t)gridDim.x * (kEigThreads * kEigLoads);
-    for (uint64_t base = ((uint64_t)blockIdx.x * (kEigThreads / 32) + warp) * (32 * kEigLoads); base < n;
-         base += stride) {
-        bool live[kEigLoads];
+    for (uint64_t base = ((uint64_t)blockIdx.x * (kEigThreads / 32) + warp) * (32 * kEigLoads);; base += stride) {
+        const bool more = base < n;
+        if (more) {
+            bool live[kEigLoads];
 #pragma unroll
-        for (uint32_t u = 0; u < kEigLoads; ++u) {
-            const uint64_t i = base + u * 32 + lane;
-            live[u] = i < n && eps.any((uint32_t)i);
-        }
+            for (uint32_t u = 0; u < kEigLoads; ++u) {
+                const uint64_t i = base + u * 32 + lane;
+                live[u] = i < n && eps.any((uint32_t)i);
+            }
 #pragma unroll
-        for (uint32_t u = 0; u < kEigLoads; ++u) {
-            const uint32_t m = __ballot_sync(0xffffffffu, live[u]);
-            if (live[u]) queue[queued + (uint32_t)__popc(m & lt)] = (uint32_t)base + u * 32 + lane;
-            queued += (uint32_t)__popc(m);
-            __syncwarp();
-            if (queued < 32) continue;
-            const uint32_t i = queue[lane];
-            queued -= 32;
-            const uint32_t rest = lane < queued ? queue[32 + lane] : 0u;
-            __syncwarp();
-            if (lane < queued) queue[lane] = rest;
-            acc += entropy_delta<MODE>(i, eps, a, b, table, h0);
+            for (uint32_t u = 0; u < kEigLoads; ++u) {
+                const uint32_t m = __ballot_sync(0xffffffffu, live[u]);
+                if (live[u]) queue[queued + (uint32_t)__popc(m & lt)] = (uint32_t)base + u * 32 + lane;
+                queued += (uint32_t)__popc(m);
+            }
             __syncwarp();
         }
+        // Full groups of 32, kEvals at a time so that their loads overlap; the
+        // rest once there is nothing more to queue. The FP64 form is long: one
+        // copy of it (unrolled over the loads, five of them missed the
+        // instruction cache).
+        constexpr uint32_t kEvals = MODE == SF_EIG_FP64 ? 1 : kEigLoads;
+        uint32_t head = 0;
+        if (kEvals > 1) {
+            while (queued - head >= 32u * kEvals) {
+                double d[kEvals];
+#pragma unroll
+                for (uint32_t u = 0; u < kEvals; ++u)
+                    d[u] = entropy_delta<MODE>(queue[head + u * 32 + lane], eps, a, b, table, h0);
+#pragma unroll
+                for (uint32_t u = 0; u < kEvals; ++u) acc += d[u];
+                head += 32u * kEvals;
+            }
+        }
+#pragma unroll 1
+        while (queued - head >= (more ? 32u : 1u)) {
+            const uint32_t cnt = min(32u, queued - head);
+            if (lane < cnt) acc += entropy_delta<MODE>(queue[head + lane], eps, a, b, table, h0);
+            head += cnt;
+        }
+        if (!more) break;
+        const uint32_t rest = queued - head;
+        const uint32_t keep = lane < rest ? queue[head + lane] : 0u;
+        __syncwarp();
+        if (lane < rest) queue[lane] = keep;
+        queued = rest;
     }
-    if (lane < queued) acc += entropy_delta<MODE>(queue[lane], eps, a, b, table, h0);
     const double total = block_sum(acc, s_warp);
     if (threadIdx.x == 0) partials[blockIdx.x] = total;
 }
