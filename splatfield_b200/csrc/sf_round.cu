@@ -581,12 +581,14 @@ int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const
             r->longest[v] = w[6];
             if (w[1] & SF_DEV_ERR_CAPACITY) over = true;
         }
+        // Also where the heads alone would fit: what a round takes does not
+        // depend on the form of its lists.
+        if (worst > (1ull << 30) - 1) return rfail(SF_ERR_CAPACITY, "intersection count exceeds 2^30-1");
         if (!over) {
             for (uint32_t v = 0; v < r->views; ++v)
                 if (r->words_host[16 * v + 3] > ((r->w[v] + 15) / 16) * ((r->h[v] + 15) / 16) / 128) r->whole[v] = 1;
             return SF_OK;
         }
-        if (worst > (1ull << 30) - 1) return rfail(SF_ERR_CAPACITY, "intersection count exceeds 2^30-1");
         r->want_cap = next_pow2(worst);
         std::fprintf(stderr, "splatfield_b200: round capacity grown to %llu intersections per view\n",
                      (unsigned long long)r->want_cap);
