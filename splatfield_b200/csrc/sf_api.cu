@@ -149,10 +149,8 @@ struct sf_scratch_t {
         cudaEvent_t status_fork = nullptr, status_join = nullptr;
         sf_view* view_dev = nullptr;
         sf_view* view_host = nullptr;   // pinned
-        const void* splats = nullptr;
-        const float* attr = nullptr;
-        const float* sh = nullptr;
-        uint32_t K = 0, n = 0, w = 0, h = 0;
+        uint64_t splats = 0;            // id of the splats captured
+        uint32_t w = 0, h = 0;
         uint64_t cap = 0;
         sf_tuning tuning{};
         bool giant = false;  // the graph includes the segmented sort
@@ -673,11 +671,7 @@ int frame_graph_capture(sf_splats sp, sf_scratch s) {
         g.exec = nullptr;
         return fail(SF_ERR_CUDA, std::string("frame graph instantiate: ") + cudaGetErrorString(e));
     }
-    g.splats = sp;
-    g.attr = sp->attr;
-    g.sh = sp->sh;
-    g.K = sp->K;
-    g.n = sp->n;
+    g.splats = sp->id;
     g.w = s->w;
     g.h = s->h;
     g.cap = s->cap;
@@ -690,9 +684,8 @@ int frame_graph_capture(sf_splats sp, sf_scratch s) {
 // tuning it was captured for changed.
 int frame_graph_ready(sf_splats sp, sf_scratch s, uint32_t w, uint32_t h) {
     auto& g = s->fg;
-    if (!g.exec || g.splats != sp || g.attr != sp->attr || g.sh != sp->sh || g.K != sp->K || g.n != sp->n ||
-        g.w != w || g.h != h || g.cap != s->cap || std::memcmp(&g.tuning, &s->tuning, sizeof(sf_tuning)) != 0 ||
-        giant_wanted(s->longest, g.giant) != g.giant)
+    if (!g.exec || g.splats != sp->id || g.w != w || g.h != h || g.cap != s->cap ||
+        std::memcmp(&g.tuning, &s->tuning, sizeof(sf_tuning)) != 0 || giant_wanted(s->longest, g.giant) != g.giant)
         return frame_graph_capture(sp, s);
     return SF_OK;
 }

@@ -1,9 +1,18 @@
 // Handle types shared by the C ABI translation units (sf_api.cu, sf_round.cu).
 #pragma once
+#include <atomic>
 #include <cstdint>
 #include <mutex>
 #include <string>
 #include "sf_internal.h"
+
+// One number per handle made, never given twice. Captured graphs keep it to
+// tell the handle they were captured with from a later one at its address,
+// whose device buffers are others.
+inline uint64_t next_handle_id() {
+    static std::atomic<uint64_t> next{1};
+    return next.fetch_add(1, std::memory_order_relaxed);
+}
 
 struct sf_ctx_t {
     int device = 0;
@@ -18,6 +27,7 @@ struct sf_ctx_t {
 };
 
 struct sf_splats_t {
+    const uint64_t id = next_handle_id();
     sf_ctx ctx = nullptr;
     uint32_t n = 0, K = 1;
     float* attr = nullptr;
@@ -35,11 +45,13 @@ struct sf_accum_t {
 };
 
 struct sf_mask_t {
+    const uint64_t id = next_handle_id();
     uint32_t w = 0, h = 0, wpr = 0;
     uint32_t* bits = nullptr;
 };
 
 struct sf_beta_t {
+    const uint64_t id = next_handle_id();
     sf_ctx ctx = nullptr;
     uint32_t n = 0;
     float *a = nullptr, *b = nullptr;

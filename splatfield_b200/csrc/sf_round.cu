@@ -123,8 +123,7 @@ struct sf_round_t {
     cudaEvent_t fork = nullptr;
     cudaGraphExec_t exec = nullptr;
     uint32_t graph_kernels = 0;  // kernel nodes of exec
-    const void* g_splats = nullptr;
-    const void* g_beta = nullptr;
+    uint64_t g_splats = 0, g_beta = 0;  // ids (0: none)
     int g_mode = -1;
     int g_adjoint = -1;
     uint32_t g_lanes = 0, g_build = 0, g_order = 0, g_split = 0, g_radix = 0;
@@ -138,9 +137,9 @@ struct sf_round_t {
     // 2.22 ms with heads whose tails some tiles want). g_whole: as
     // captured.
     std::vector<uint8_t> whole, g_whole;
-    const void* whole_splats = nullptr;
+    uint64_t whole_splats = 0;  // id
     uint32_t chunks = 1;
-    std::vector<const sf_mask_t*> g_masks;
+    std::vector<uint64_t> g_masks;  // ids (0: no mask)
 };
 
 namespace {
@@ -477,6 +476,12 @@ cudaError_t use_dev(int dev) {
     return cur == dev ? cudaSuccess : cudaSetDevice(dev);
 }
 
+std::vector<uint64_t> mask_ids(const sf_round_t* r) {
+    std::vector<uint64_t> ids;
+    for (const sf_mask_t* m : r->masks) ids.push_back(m ? m->id : 0);
+    return ids;
+}
+
 // Capture the whole round into r->exec.
 int build_graph(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, int mode) {
     graph_drop(r);
@@ -517,8 +522,8 @@ int build_graph(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, int
         r->exec = nullptr;
         return rfail(SF_ERR_CUDA, std::string("round graph instantiate: ") + cudaGetErrorString(e));
     }
-    r->g_splats = sp;
-    r->g_beta = beta;
+    r->g_splats = sp->id;
+    r->g_beta = beta ? beta->id : 0;
     r->g_mode = mode;
     r->g_adjoint = (int)r->adjoint;
     r->g_lanes = (uint32_t)r->lanes.size();
@@ -526,7 +531,7 @@ int build_graph(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, int
     r->g_order = r->tuning.raster_order;
     r->g_split = r->tuning.raster_split;
     r->g_radix = r->tuning.radix_bits;
-    r->g_masks = r->masks;
+    r->g_masks = mask_ids(r);
     for (uint32_t v = 0; v < r->views; ++v) r->g_giant[v] = giant_wanted(r->longest[v], r->g_giant[v]);
     r->g_whole = r->whole;
     return SF_OK;
@@ -543,20 +548,20 @@ bool giant_changed(const sf_round_t* r) {
 int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const sf_camera* cams, int mode,
               cudaStream_t user) {
     for (uint32_t v = 0; v < r->views; ++v) view_for_camera(cams[v], r->w[v], r->h[v], &r->views_host[v]);
-    if (r->whole_splats != sp) {
+    if (r->whole_splats != sp->id) {
         r->whole.assign(r->views, 0);
-        r->whole_splats = sp;
+        r->whole_splats = sp->id;
     }
     for (int attempt = 0; attempt < 4; ++attempt) {
         const uint32_t lanes = std::max(1u, std::min(r->tuning.lanes ? r->tuning.lanes : 4u, r->views));
         if (r->lanes.size() != lanes || r->lanes[0].cap < r->want_cap) {
             RF_CK(lanes_build(r, lanes, std::max<uint64_t>(r->want_cap, r->lanes.empty() ? 1024 : r->lanes[0].cap)));
         }
-        if (!r->exec || r->g_splats != sp || r->g_beta != beta || r->g_mode != mode ||
+        if (!r->exec || r->g_splats != sp->id || r->g_beta != (beta ? beta->id : 0) || r->g_mode != mode ||
             r->g_adjoint != (int)r->adjoint ||
             r->g_build != r->tuning.isect_build ||
             r->g_order != r->tuning.raster_order || r->g_split != r->tuning.raster_split ||
-            r->g_radix != r->tuning.radix_bits || r->g_masks != r->masks || r->g_whole != r->whole ||
+            r->g_radix != r->tuning.radix_bits || r->g_masks != mask_ids(r) || r->g_whole != r->whole ||
             giant_changed(r)) {
             const int rc = build_graph(r, sp, beta, mode);
             if (rc != SF_OK) return rc;
