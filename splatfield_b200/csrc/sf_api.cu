@@ -139,8 +139,8 @@ struct sf_scratch_t {
     bool lazy = false;
     uint32_t lazy_min = 0;  // lists longer than this are ordered in the raster
     SortStreams sort_streams;  // concurrent per-tile sort classes inside the frame graph
-    // Frame graph (binned RGB frames): one capture per (splats, size,
-    // capacity, tuning), replayed with the camera copied in by its first node.
+    // Frame graph (binned RGB frames): one capture per splats, tuning and set
+    // of buffers, replayed with the camera copied in before it.
     struct FrameGraph {
         cudaGraphExec_t exec = nullptr;
         uint32_t kernels = 0;           // kernel nodes of exec
@@ -150,8 +150,6 @@ struct sf_scratch_t {
         sf_view* view_dev = nullptr;
         sf_view* view_host = nullptr;   // pinned
         uint64_t splats = 0;            // id of the splats captured
-        uint32_t w = 0, h = 0;
-        uint64_t cap = 0;
         sf_tuning tuning{};
         bool giant = false;  // the graph includes the segmented sort
         // Frames to host memory in a batch: each image is copied out of the
@@ -227,7 +225,14 @@ cudaError_t ensure_lut(sf_ctx ctx) {
     return cudaMemcpy(ctx->lut, t.data(), t.size() * 4, cudaMemcpyHostToDevice);
 }
 
+// The captured frame holds the buffers' addresses: it goes before they do.
+void frame_graph_drop(sf_scratch s) {
+    if (s->fg.exec) cudaGraphExecDestroy(s->fg.exec);
+    s->fg.exec = nullptr;
+}
+
 void scratch_free_frame(sf_scratch s) {
+    frame_graph_drop(s);
     dfree(s->depth_keys); dfree(s->tile_counts); dfree(s->bbox); dfree(s->geo0); dfree(s->geo1);
     dfree(s->color); dfree(s->ext); dfree(s->keys_a); dfree(s->keys_b); dfree(s->order_a); dfree(s->order_b);
     dfree(s->offsets); dfree(s->scan_tmp); dfree(s->tile_start); dfree(s->bitmap);
@@ -263,6 +268,7 @@ cudaError_t ensure_sort_tmp(sf_scratch s, size_t bytes) {
 
 cudaError_t grow_isects(sf_scratch s, uint64_t want) {
     if (want <= s->cap && s->tid_e) return cudaSuccess;
+    frame_graph_drop(s);
     const uint64_t cap = std::min<uint64_t>(std::max<uint64_t>(next_pow2(want), 1024), kMaxIsects + 1);
     dfree(s->tid_e); dfree(s->gid_e); dfree(s->tid_a);
     s->gid_a = nullptr;
@@ -581,10 +587,7 @@ constexpr uint32_t kFrameRing = 4096;  // frames whose status words the ring hol
 
 int frame_graph_capture(sf_splats sp, sf_scratch s) {
     auto& g = s->fg;
-    if (g.exec) {
-        cudaGraphExecDestroy(g.exec);
-        g.exec = nullptr;
-    }
+    frame_graph_drop(s);
     if (!g.stream) SF_CK(cudaStreamCreateWithFlags(&g.stream, cudaStreamNonBlocking));
     if (!g.status) SF_CK(cudaStreamCreateWithFlags(&g.status, cudaStreamNonBlocking));
     if (!g.status_fork) SF_CK(cudaEventCreateWithFlags(&g.status_fork, cudaEventDisableTiming));
@@ -672,19 +675,16 @@ int frame_graph_capture(sf_splats sp, sf_scratch s) {
         return fail(SF_ERR_CUDA, std::string("frame graph instantiate: ") + cudaGetErrorString(e));
     }
     g.splats = sp->id;
-    g.w = s->w;
-    g.h = s->h;
-    g.cap = s->cap;
     g.tuning = s->tuning;
     g.giant = giant;
     return SF_OK;
 }
 
-// (Re)captures the frame graph when the splats, image size, capacity or
+// (Re)captures the frame graph when the scratch's buffers, the splats or the
 // tuning it was captured for changed.
-int frame_graph_ready(sf_splats sp, sf_scratch s, uint32_t w, uint32_t h) {
+int frame_graph_ready(sf_splats sp, sf_scratch s) {
     auto& g = s->fg;
-    if (!g.exec || g.splats != sp->id || g.w != w || g.h != h || g.cap != s->cap ||
+    if (!g.exec || g.splats != sp->id ||
         std::memcmp(&g.tuning, &s->tuning, sizeof(sf_tuning)) != 0 || giant_wanted(s->longest, g.giant) != g.giant)
         return frame_graph_capture(sp, s);
     return SF_OK;
@@ -714,7 +714,7 @@ int frame_graph_render(sf_splats sp, sf_scratch s, const sf_camera* cam, uint32_
                        cudaStream_t st, uint32_t* host_out) {
     auto& g = s->fg;
     for (int attempt = 0; attempt < 4; ++attempt) {
-        const int rc = frame_graph_ready(sp, s, w, h);
+        const int rc = frame_graph_ready(sp, s);
         if (rc != SF_OK) return rc;
         view_for_camera(*cam, w, h, g.view_host);
         SF_CK(cudaMemcpyAsync(g.view_dev, g.view_host, sizeof(sf_view), cudaMemcpyHostToDevice, st));
@@ -794,7 +794,7 @@ int twin_ready(sf_splats sp, sf_scratch s, uint32_t w, uint32_t h) {
     if (!s->twin_stream) SF_CK(cudaStreamCreateWithFlags(&s->twin_stream, cudaStreamNonBlocking));
     if (!s->fork) SF_CK(cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming));
     if (!s->join) SF_CK(cudaEventCreateWithFlags(&s->join, cudaEventDisableTiming));
-    return frame_graph_ready(sp, t, w, h);
+    return frame_graph_ready(sp, t);
 }
 
 // Copies the status words that run [first, end) of a camera path saved to
@@ -835,7 +835,7 @@ int frames_graph_render(sf_splats sp, sf_scratch s, const sf_camera* cams, uint3
     auto& g = s->fg;
     const size_t img = (size_t)w * h;
     bool two = count >= 2 && s->tuning.frame_pipes != 1;
-    int rc = frame_graph_ready(sp, s, w, h);
+    int rc = frame_graph_ready(sp, s);
     if (rc != SF_OK) return rc;
     if (two && (rc = twin_ready(sp, s, w, h)) != SF_OK) {
         if (rc != SF_ERR_NOMEM) return rc;
@@ -1151,7 +1151,6 @@ int sf_scratch_destroy(sf_scratch s) {
     dfree(s->words);  // and the stats behind them
     if (s->host_words) cudaFreeHost(s->host_words);
     sort_streams_destroy(&s->sort_streams);
-    if (s->fg.exec) cudaGraphExecDestroy(s->fg.exec);
     if (s->fg.stream) cudaStreamDestroy(s->fg.stream);
     if (s->fg.status) cudaStreamDestroy(s->fg.status);
     if (s->fg.status_fork) cudaEventDestroy(s->fg.status_fork);
