@@ -329,6 +329,7 @@ constexpr uint32_t kHeadTarget = 2048;   // pairs aimed at
 constexpr uint32_t kHeadKeep = 3072;     // lists estimated no longer than this are not cut
 constexpr uint32_t kHeadMinSplats = 640000, kHeadMinTiles = 1024, kHeadSplats = 512;
 constexpr uint32_t kHeadMaxTiles = 12288;  // limits and counters of a block: 96 KB
+constexpr unsigned long long kMaxPairs = (1ull << 30) - 1;  // of a frame's whole lists
 
 __global__ __launch_bounds__(256) void head_sample_kernel(const uint2* __restrict__ bbox,
                                                           const uint32_t* __restrict__ depth_keys, uint32_t n,
@@ -455,13 +456,23 @@ __device__ __forceinline__ void for_each_tail_pair(const uint2* __restrict__ bbo
     }
 }
 
+// A view whose heads outgrew the capacity is drawn again after it has grown,
+// and one past the intersection limit is refused: no tails then. (A cut leaves
+// the tiles past it with empty heads, so all of them are listed, and their
+// tails are every pair they have: such an attempt at a round of 3M splats took
+// 6.4 to 7.5 ms, the round itself 5.0 to 5.6.)
+__device__ __forceinline__ bool heads_lost(const HeadState& h, uint32_t capacity, const unsigned long long* total_all) {
+    return *reinterpret_cast<const unsigned long long*>(h.ctrl + 2) > capacity || *total_all > kMaxPairs;
+}
+
 // Counts and slots go through a counter per tile in shared memory: a listed
 // tile's tail may hold thousands of pairs, and as many atomics on one address.
 constexpr uint32_t kTailThreads = 512;
 __global__ __launch_bounds__(kTailThreads) void tail_count_kernel(const uint2* __restrict__ bbox,
                                                                   const uint32_t* __restrict__ depth_keys, uint32_t n,
-                                                                  uint32_t tiles_x, uint32_t tiles, HeadState h) {
-    if (h.ctrl[0] == 0) return;
+                                                                  uint32_t tiles_x, uint32_t tiles, uint32_t capacity,
+                                                                  const unsigned long long* total_all, HeadState h) {
+    if (h.ctrl[0] == 0 || heads_lost(h, capacity, total_all)) return;
     extern __shared__ uint32_t s_n[];
     __shared__ uint32_t s_bits[kHeadMaxTiles / 32];
     for (uint32_t w = threadIdx.x; w < (tiles + 31) / 32; w += kTailThreads) s_bits[w] = h.bits[w];
@@ -474,35 +485,45 @@ __global__ __launch_bounds__(kTailThreads) void tail_count_kernel(const uint2* _
         if (s_n[t]) atomicAdd(h.tail_n + t, s_n[t]);
 }
 
-// First slots of the listed tiles' tails, after the heads.
-// *listed = how many they are.
-__global__ __launch_bounds__(1024) void tail_plan_kernel(HeadState h, uint32_t capacity, uint32_t* listed) {
+// First slots of the listed tiles' tails, after the heads; *listed = how many
+// they are, *wanted the pairs of heads and tails together. ctrl[1]: the tails
+// are left out (heads_lost, or they do not fit).
+__global__ __launch_bounds__(1024) void tail_plan_kernel(HeadState h, uint32_t capacity,
+                                                         const unsigned long long* total_all, uint32_t* err,
+                                                         uint32_t* listed, uint32_t* wanted) {
     __shared__ uint32_t s32[32];
-    const uint32_t count = h.ctrl[0];
-    if (threadIdx.x == 0) *listed = count;
     const unsigned long long heads = *reinterpret_cast<const unsigned long long*>(h.ctrl + 2);
-    uint32_t base = (uint32_t)(heads < capacity ? heads : capacity);
-    for (uint32_t i0 = 0; i0 < count; i0 += 1024) {
-        const uint32_t i = i0 + threadIdx.x;
-        const uint32_t t = i < count ? h.list[i] : 0u;
-        const uint32_t c = i < count ? h.tail_n[t] : 0u;
-        uint32_t total;
-        const uint32_t at = base + block_scan<1024>(c, s32, total);
-        if (i < count) {
-            // Past the capacity the frame is drawn again after it has grown.
-            h.tail_start[t] = h.tail_at[t] = min(at, capacity);
-            h.tail_n[t] = at < capacity ? min(c, capacity - at) : 0u;
+    const bool lost = heads_lost(h, capacity, total_all);
+    const uint32_t count = h.ctrl[0];
+    // Not lost: heads and tails are part of the whole lists, so every sum is
+    // within kMaxPairs.
+    uint32_t base = (uint32_t)(heads < 0xffffffffull ? heads : 0xffffffffull);
+    if (!lost) {
+        for (uint32_t i0 = 0; i0 < count; i0 += 1024) {
+            const uint32_t i = i0 + threadIdx.x;
+            const uint32_t t = i < count ? h.list[i] : 0u;
+            const uint32_t c = i < count ? h.tail_n[t] : 0u;
+            uint32_t total;
+            const uint32_t at = base + block_scan<1024>(c, s32, total);
+            if (i < count) h.tail_start[t] = h.tail_at[t] = at;
+            base += total;
         }
-        base += total;
+    }
+    if (threadIdx.x == 0) {
+        *listed = count;
+        *wanted = base;
+        if (lost || base > capacity) {
+            h.ctrl[1] = 1u;
+            atomicOr(err, SF_DEV_ERR_CAPACITY);
+        }
     }
 }
 
 __global__ __launch_bounds__(kTailThreads) void tail_place_kernel(const uint2* __restrict__ bbox,
                                                                   const uint32_t* __restrict__ depth_keys, uint32_t n,
                                                                   uint32_t tiles_x, uint32_t tiles, uint32_t capacity,
-                                                                  uint2* __restrict__ pairs, uint32_t* err,
-                                                                  HeadState h) {
-    if (h.ctrl[0] == 0) return;
+                                                                  uint2* __restrict__ pairs, HeadState h) {
+    if (h.ctrl[0] == 0 || h.ctrl[1]) return;
     extern __shared__ uint32_t s_n[];
     __shared__ uint32_t s_bits[kHeadMaxTiles / 32];
     for (uint32_t w = threadIdx.x; w < (tiles + 31) / 32; w += kTailThreads) s_bits[w] = h.bits[w];
@@ -517,8 +538,7 @@ __global__ __launch_bounds__(kTailThreads) void tail_place_kernel(const uint2* _
     __syncthreads();
     for_each_tail_pair(bbox, depth_keys, n, tiles_x, s_bits, h.limit, [&](uint32_t t, uint32_t key, uint32_t s) {
         const uint32_t slot = atomicAdd(s_n + t, 1u);
-        if (slot < capacity) pairs[slot] = make_uint2(key, s);
-        else atomicOr(err, SF_DEV_ERR_CAPACITY);
+        if (slot < capacity) pairs[slot] = make_uint2(key, s);  // always: the plan fits
     });
 }
 
@@ -1492,6 +1512,8 @@ cudaError_t launch_bin_place(const uint2* bbox, const uint32_t* depth_keys, uint
     return e;
 }
 
+uint64_t heads_pairs(uint32_t tiles) { return (uint64_t)tiles * kHeadTarget; }
+
 bool heads_wanted(uint32_t n, uint32_t tiles) {
     return n >= kHeadMinSplats && tiles >= kHeadMinTiles && tiles <= kHeadMaxTiles && n / kHeadSplats >= tiles;
 }
@@ -1537,10 +1559,10 @@ cudaError_t launch_tail_place(const uint2* bbox, const uint32_t* depth_keys, uin
     cudaError_t e = smem_opt_in((const void*)tail_count_kernel, smem, kTailSmem);
     if (e == cudaSuccess) e = smem_opt_in((const void*)tail_place_kernel, smem, kTailSmem);
     if (e != cudaSuccess) return e;
-    tail_count_kernel<<<blocks, kTailThreads, smem, st>>>(bbox, depth_keys, n, tiles_x, tiles, h);
-    tail_plan_kernel<<<1, 1024, 0, st>>>(h, capacity, words + 3);
-    tail_place_kernel<<<blocks, kTailThreads, smem, st>>>(bbox, depth_keys, n, tiles_x, tiles, capacity, pairs, words + 1,
-                                                          h);
+    const auto* total_all = reinterpret_cast<const unsigned long long*>(words + 4);
+    tail_count_kernel<<<blocks, kTailThreads, smem, st>>>(bbox, depth_keys, n, tiles_x, tiles, capacity, total_all, h);
+    tail_plan_kernel<<<1, 1024, 0, st>>>(h, capacity, total_all, words + 1, words + 3, words + 2);
+    tail_place_kernel<<<blocks, kTailThreads, smem, st>>>(bbox, depth_keys, n, tiles_x, tiles, capacity, pairs, h);
     note_launches(3);
     return cudaGetLastError();
 }

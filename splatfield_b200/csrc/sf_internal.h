@@ -225,7 +225,9 @@ constexpr uint32_t kHeadSamples = 256;  // sampled keys kept per tile
 struct HeadState {
     // Cleared before each view, one block of zero_words: ctrl, sampled,
     // tail_n, bits.
-    uint32_t* ctrl = nullptr;     // [8]: [0] tiles in `list`, [2..3] pairs placed in heads (u64)
+    // [8]: [0] tiles in `list`, [1] tails left out (the capacity is too
+    // small), [2..3] pairs of the heads (u64)
+    uint32_t* ctrl = nullptr;
     uint32_t* sampled = nullptr;  // [8 * tiles]: sampled pairs, a counter per 32 bytes
     uint32_t* tail_n = nullptr;   // [tiles]: tail pairs of a listed tile
     uint32_t* bits = nullptr;     // [ceil(tiles / 32)]: listed tiles
@@ -237,6 +239,8 @@ struct HeadState {
     uint32_t* list = nullptr;        // [tiles]: tiles whose pixels want their tail
     float* t = nullptr;              // [pixels]: transmittance after the head (tiles with a tail)
 };
+// Pairs that the heads of `tiles` tiles aim at.
+uint64_t heads_pairs(uint32_t tiles);
 // Whether a view of `tiles` tiles over n splats takes depth-limited lists.
 bool heads_wanted(uint32_t n, uint32_t tiles);
 // limit[t] from every 32nd splat's boxes and keys.
@@ -250,8 +254,10 @@ cudaError_t launch_head_count(const uint2* bbox, const uint32_t* depth_keys, uin
 cudaError_t launch_head_place(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
                               uint32_t tiles, uint32_t chunks, const uint32_t* hist, const uint32_t* tile_start,
                               uint32_t capacity, uint2* pairs, uint32_t* err, const HeadState& h, cudaStream_t st);
-// The tails of the listed tiles, unsorted, after the heads in `pairs`; words[1]
-// as in launch_head_place, words[3] = listed tiles.
+// The tails of the listed tiles, unsorted, after the heads in `pairs`, when
+// both fit the capacity; words[1] as in launch_head_place, words[2] = pairs of
+// heads and wanted tails (of the heads alone when these do not fit), words[3] =
+// listed tiles; words[4..5] is the total of the whole lists.
 cudaError_t launch_tail_place(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
                               uint32_t tiles, uint32_t capacity, uint2* pairs, uint32_t* words, const HeadState& h,
                               cudaStream_t st);

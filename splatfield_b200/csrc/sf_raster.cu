@@ -705,7 +705,7 @@ __global__ __launch_bounds__(NT) void raster_kernel(RasterArgs a) {
 // The tails of the listed tiles, a CTA each in turn.
 template <int MODE>
 __global__ __launch_bounds__(256) void raster_tails_kernel(RasterArgs a) {
-    const uint32_t count = *a.head_ctrl;
+    const uint32_t count = a.head_ctrl[1] ? 0u : a.head_ctrl[0];
     for (uint32_t i = blockIdx.x; i < count; i += gridDim.x) {
         raster_tile<MODE, true, false, false, true, true, 256>(a, a.head_list[i], 0);
         __syncthreads();

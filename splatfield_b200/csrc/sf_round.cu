@@ -101,7 +101,9 @@ struct sf_round_t {
     std::vector<RoundLane> lanes;
     sf_view* views_dev = nullptr;
     sf_view* views_host = nullptr;  // pinned
-    uint32_t* words = nullptr;      // [views][16]: 0 visible, 1 err, 2 n32, 3 tiles past their heads, 4..5 total u64, 6..14 binned stats
+    // [views][16]: 0 visible, 1 err, 2 n32 (heads: their pairs and the wanted
+    // tails'), 3 tiles past their heads, 4..5 total u64, 6..15 binned stats
+    uint32_t* words = nullptr;
     uint32_t* words_host = nullptr; // pinned
     double* eig_dev = nullptr;
     double* eig_host = nullptr;     // pinned
@@ -137,6 +139,7 @@ struct sf_round_t {
     // 2.22 ms with heads whose tails some tiles want). g_whole: as
     // captured.
     std::vector<uint8_t> whole, g_whole;
+    std::vector<uint8_t> g_heads;  // views captured with depth-limited lists
     uint64_t whole_splats = 0;  // id
     uint32_t chunks = 1;
     std::vector<uint64_t> g_masks;  // ids (0: no mask)
@@ -157,7 +160,7 @@ void lane_free(RoundLane& L) {
     dfree(L.giant.ctrl); dfree(L.giant.sel); dfree(L.giant.mm); dfree(L.giant.hist);
     dfree(L.giant.taken); dfree(L.giant.segs);
     L.giant.lists = L.giant.seg_cap = 0;
-    dfree(L.head.ctrl); dfree(L.head.keys); dfree(L.head.limit); dfree(L.head.t);
+    dfree(L.head.ctrl);
     L.head = HeadState();
     sort_streams_destroy(&L.sort_streams);
     if (L.stream) cudaStreamDestroy(L.stream);
@@ -201,16 +204,17 @@ cudaError_t lane_alloc(sf_round_t* r, RoundLane& L, uint64_t cap) {
     if (head_tiles) {
         HeadState& H = L.head;
         H.zero_words = 8 + 9 * (size_t)head_tiles + (head_tiles + 31) / 32;
-        RA(H.ctrl, H.zero_words);
+        // One allocation: a lane's first call is mostly these.
+        RA(H.ctrl, H.zero_words + (kHeadSamples + 4) * (size_t)head_tiles + head_pixels);
         H.sampled = H.ctrl + 8;
         H.tail_n = H.sampled + 8 * (size_t)head_tiles;
         H.bits = H.tail_n + head_tiles;
-        RA(H.keys, (size_t)head_tiles * kHeadSamples);
-        RA(H.limit, 4 * (size_t)head_tiles);
+        H.keys = H.ctrl + H.zero_words;
+        H.limit = H.keys + (size_t)head_tiles * kHeadSamples;
         H.tail_start = H.limit + head_tiles;
         H.tail_at = H.tail_start + head_tiles;
         H.list = H.tail_at + head_tiles;
-        RA(H.t, head_pixels);
+        H.t = reinterpret_cast<float*>(H.list + head_tiles);
     }
 #undef RA
     if ((e = cudaMalloc(&L.scan_tmp, scan_temp_bytes(std::max(n, r->max_tiles + 1)))) != cudaSuccess) return e;
@@ -382,6 +386,13 @@ cudaError_t adjoint_and_eig(sf_round_t* r, RoundLane& L, uint32_t v, uint32_t tx
     return cudaSuccess;
 }
 
+// Whether view v takes depth-limited lists.
+bool view_heads(const sf_round_t* r, uint32_t v) {
+    const uint32_t tiles = ((r->w[v] + 15) / 16) * ((r->h[v] + 15) / 16);
+    return r->tuning.isect_build == SF_ISECTS_BINNED && r->max_tiles <= kBinMaxTiles &&
+           (r->adjoint || r->tuning.raster_order == SF_ORDER_SORTED) && !r->whole[v] && heads_wanted(r->n, tiles);
+}
+
 // One view's pipeline on lane L's stream.
 cudaError_t enqueue_view(sf_round_t* r, RoundLane& L, uint32_t v, const sf_splats_t& sp,
                          const float* beta_a, const float* beta_b, const float* lut, int mode) {
@@ -399,9 +410,7 @@ cudaError_t enqueue_view(sf_round_t* r, RoundLane& L, uint32_t v, const sf_splat
     if ((e = launch_project(dummy, sp.attr, sp.geom, sp.sh, n, sp.K, po, st, r->views_dev + v)) != cudaSuccess) return e;
     const uint32_t *tids = nullptr, *gids = nullptr;
     const uint2* lazy_pairs = nullptr;
-    const bool heads = r->tuning.isect_build == SF_ISECTS_BINNED && L.hist && L.head.ctrl &&
-                       (r->adjoint || r->tuning.raster_order == SF_ORDER_SORTED) && !r->whole[v] &&
-                       heads_wanted(n, tiles);
+    const bool heads = view_heads(r, v);
     if (heads) {
         // Only the nearest pairs of each tile are counted, placed and sorted;
         // words[4..5] gets the pairs of the whole lists.
@@ -534,6 +543,8 @@ int build_graph(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, int
     r->g_masks = mask_ids(r);
     for (uint32_t v = 0; v < r->views; ++v) r->g_giant[v] = giant_wanted(r->longest[v], r->g_giant[v]);
     r->g_whole = r->whole;
+    r->g_heads.resize(r->views);
+    for (uint32_t v = 0; v < r->views; ++v) r->g_heads[v] = view_heads(r, v);
     return SF_OK;
 }
 
@@ -552,7 +563,8 @@ int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const
         r->whole.assign(r->views, 0);
         r->whole_splats = sp->id;
     }
-    for (int attempt = 0; attempt < 4; ++attempt) {
+    // Heads may outgrow the capacity, then the tails that they leave.
+    for (int attempt = 0; attempt < 6; ++attempt) {
         const uint32_t lanes = std::max(1u, std::min(r->tuning.lanes ? r->tuning.lanes : 4u, r->views));
         if (r->lanes.size() != lanes || r->lanes[0].cap < r->want_cap) {
             RF_CK(lanes_build(r, lanes, std::max<uint64_t>(r->want_cap, r->lanes.empty() ? 1024 : r->lanes[0].cap)));
@@ -575,7 +587,7 @@ int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const
         RF_CK(cudaGraphLaunch(r->exec, r->main));
         note_launches(r->graph_kernels);
         RF_CK(cudaStreamSynchronize(r->main));
-        uint64_t worst = 0;
+        uint64_t worst = 0, need = 0;
         bool over = false;
         for (uint32_t v = 0; v < r->views; ++v) {
             const uint32_t* w = r->words_host + 16 * v;
@@ -585,6 +597,8 @@ int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const
             worst = std::max(worst, total);
             r->longest[v] = w[6];
             if (w[1] & SF_DEV_ERR_CAPACITY) over = true;
+            // The heads' cuts move a little from run to run (their sample does).
+            need = std::max<uint64_t>(need, r->g_heads[v] ? w[2] + w[2] / 16 : total);
         }
         // Also where the heads alone would fit: what a round takes does not
         // depend on the form of its lists.
@@ -594,7 +608,7 @@ int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const
                 if (r->words_host[16 * v + 3] > ((r->w[v] + 15) / 16) * ((r->h[v] + 15) / 16) / 128) r->whole[v] = 1;
             return SF_OK;
         }
-        r->want_cap = next_pow2(worst);
+        r->want_cap = std::max(r->want_cap, std::min<uint64_t>(next_pow2(need), 1ull << 30));
         std::fprintf(stderr, "splatfield_b200: round capacity grown to %llu intersections per view\n",
                      (unsigned long long)r->want_cap);
     }
@@ -640,13 +654,20 @@ int sf_round_create(sf_ctx ctx, uint32_t total, uint32_t n_views, const uint32_t
     r->h.assign(heights, heights + n_views);
     r->longest.assign(n_views, 0u);
     r->g_giant.assign(n_views, 0u);
+    uint64_t heads = 0;  // pairs of the largest view's heads
     for (uint32_t v = 0; v < n_views; ++v) {
-        r->max_tiles = std::max(r->max_tiles, ((widths[v] + 15) / 16) * ((heights[v] + 15) / 16));
+        const uint32_t tiles = ((widths[v] + 15) / 16) * ((heights[v] + 15) / 16);
+        r->max_tiles = std::max(r->max_tiles, tiles);
+        if (heads_wanted(total, tiles)) heads = std::max(heads, heads_pairs(tiles));
     }
     r->eig_blocks = eig_blocks(total, ctx->sm_count);
     r->chunks = bin_chunks(total, ctx->sm_count);
     r->tuning.lanes = 4;
-    r->want_cap = std::min<uint64_t>((uint64_t)r->max_tiles * total, 1ull << 22);
+    // A 1024x1024 view of 3M splats has heads of 4.6M to 6.9M pairs: room for
+    // what its heads aim at saves the first round a lost attempt and a second
+    // allocation. (Views with heads have 512 splats a tile or more, so that is
+    // at most 4 pairs a splat, 8 rounded up.)
+    r->want_cap = std::max(std::min<uint64_t>((uint64_t)r->max_tiles * total, 1ull << 22), next_pow2(heads));
     cudaError_t e = cudaStreamCreateWithFlags(&r->main, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&r->fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = dalloc(&r->views_dev, n_views);
