@@ -350,7 +350,8 @@ __global__ __launch_bounds__(256) void head_sample_kernel(const uint2* __restric
 }
 
 // A warp per tile: the rank-th smallest of its sampled keys, by bisection.
-__global__ __launch_bounds__(256) void head_pick_kernel(uint32_t tiles, HeadState h) {
+// *longest: at least the longest whole list, as the sample has it.
+__global__ __launch_bounds__(256) void head_pick_kernel(uint32_t tiles, HeadState h, uint32_t* longest) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t t = blockIdx.x * 8u + (threadIdx.x >> 5);
     if (t >= tiles) return;
@@ -381,7 +382,11 @@ __global__ __launch_bounds__(256) void head_pick_kernel(uint32_t tiles, HeadStat
         }
         limit = lo;
     }
-    if (lane == 0) h.limit[t] = limit;
+    if (lane == 0) {
+        h.limit[t] = limit;
+        // Only lists that the segmented sort may concern.
+        if (c >= kGiantMinList / 2 / kHeadStride) atomicMax(longest, min(c, 0xffffffffu / kHeadStride) * kHeadStride);
+    }
 }
 
 __global__ __launch_bounds__(kBinThreads, 2) void head_count_kernel(
@@ -1519,10 +1524,10 @@ bool heads_wanted(uint32_t n, uint32_t tiles) {
 }
 
 cudaError_t launch_head_limits(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
-                               uint32_t tiles, const HeadState& h, cudaStream_t st) {
+                               uint32_t tiles, const HeadState& h, uint32_t* longest, cudaStream_t st) {
     const uint32_t sampled = (n + kHeadStride - 1) / kHeadStride;
     head_sample_kernel<<<(sampled + 255) / 256, 256, 0, st>>>(bbox, depth_keys, n, tiles_x, h);
-    head_pick_kernel<<<(tiles + 7) / 8, 256, 0, st>>>(tiles, h);
+    head_pick_kernel<<<(tiles + 7) / 8, 256, 0, st>>>(tiles, h, longest);
     note_launches(2);
     return cudaGetLastError();
 }

@@ -243,9 +243,10 @@ struct HeadState {
 uint64_t heads_pairs(uint32_t tiles);
 // Whether a view of `tiles` tiles over n splats takes depth-limited lists.
 bool heads_wanted(uint32_t n, uint32_t tiles);
-// limit[t] from every 32nd splat's boxes and keys.
+// limit[t] from every 32nd splat's boxes and keys; *longest = max(*longest, the
+// longest whole list by that sample), where it is of the segmented sort's lengths.
 cudaError_t launch_head_limits(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,
-                               uint32_t tiles, const HeadState& h, cudaStream_t st);
+                               uint32_t tiles, const HeadState& h, uint32_t* longest, cudaStream_t st);
 // launch_bin_count / launch_bin_place over the pairs of the heads; *total_all
 // += the pairs of the whole lists.
 cudaError_t launch_head_count(const uint2* bbox, const uint32_t* depth_keys, uint32_t n, uint32_t tiles_x,

@@ -102,7 +102,8 @@ struct sf_round_t {
     sf_view* views_dev = nullptr;
     sf_view* views_host = nullptr;  // pinned
     // [views][16]: 0 visible, 1 err, 2 n32 (heads: their pairs and the wanted
-    // tails'), 3 tiles past their heads, 4..5 total u64, 6..15 binned stats
+    // tails'), 3 tiles past their heads, 4..5 total u64, 6 longest list, 7 longest
+    // whole list (heads: by their sample), 8..15 tiles of each size class
     uint32_t* words = nullptr;
     uint32_t* words_host = nullptr; // pinned
     double* eig_dev = nullptr;
@@ -129,8 +130,9 @@ struct sf_round_t {
     int g_mode = -1;
     int g_adjoint = -1;
     uint32_t g_lanes = 0, g_build = 0, g_order = 0, g_split = 0, g_radix = 0;
-    // Per view: the longest tile list of the last round, and whether the
-    // graph includes the segmented sort of the longest lists for the view.
+    // Per view: the longest whole tile list of the last round (of one with
+    // heads, as their sample has it), and whether the graph includes the
+    // segmented sort of the longest lists for the view.
     std::vector<uint32_t> longest;
     std::vector<uint8_t> g_giant;
     // Views whose heads left more than one in 128 of their tiles unsaturated
@@ -393,6 +395,11 @@ bool view_heads(const sf_round_t* r, uint32_t v) {
            (r->adjoint || r->tuning.raster_order == SF_ORDER_SORTED) && !r->whole[v] && heads_wanted(r->n, tiles);
 }
 
+// Whether view v takes the segmented sort (heads do not).
+bool view_giant(const sf_round_t* r, uint32_t v) {
+    return !view_heads(r, v) && giant_wanted(r->longest[v], r->g_giant[v]);
+}
+
 // One view's pipeline on lane L's stream.
 cudaError_t enqueue_view(sf_round_t* r, RoundLane& L, uint32_t v, const sf_splats_t& sp,
                          const float* beta_a, const float* beta_b, const float* lut, int mode) {
@@ -418,7 +425,7 @@ cudaError_t enqueue_view(sf_round_t* r, RoundLane& L, uint32_t v, const sf_splat
         unsigned long long* placed = reinterpret_cast<unsigned long long*>(H.ctrl + 2);
         uint2* pairs = reinterpret_cast<uint2*>(L.tid_a);
         if ((e = cudaMemsetAsync(H.ctrl, 0, 4 * H.zero_words, st)) != cudaSuccess) return e;
-        if ((e = launch_head_limits(L.bbox, L.keys, n, tx, tiles, H, st)) != cudaSuccess) return e;
+        if ((e = launch_head_limits(L.bbox, L.keys, n, tx, tiles, H, words + 7, st)) != cudaSuccess) return e;
         if ((e = launch_head_count(L.bbox, L.keys, n, tx, tiles, r->chunks, L.hist, H, total, st)) != cudaSuccess)
             return e;
         if ((e = launch_bin_colscan(L.hist, r->chunks, tiles, L.cnt, L.lists, words, st)) != cudaSuccess) return e;
@@ -451,8 +458,7 @@ cudaError_t enqueue_view(sf_round_t* r, RoundLane& L, uint32_t v, const sf_splat
             if (order == SF_ORDER_HYBRID) grids[kSortClasses - 1] = 0;
             if ((e = launch_tile_sorts(grids, L.lists, words, tiles, L.tile_start, (uint32_t)L.cap, pairs, L.gid_e,
                                        nullptr, L.tid_e, r->sm_count, st, &L.sort_streams,
-                                       giant_wanted(r->longest[v], r->g_giant[v]) ? &L.giant : nullptr)) !=
-                cudaSuccess)
+                                       view_giant(r, v) ? &L.giant : nullptr)) != cudaSuccess)
                 return e;
             gids = L.gid_e;
         }
@@ -541,7 +547,7 @@ int build_graph(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, int
     r->g_split = r->tuning.raster_split;
     r->g_radix = r->tuning.radix_bits;
     r->g_masks = mask_ids(r);
-    for (uint32_t v = 0; v < r->views; ++v) r->g_giant[v] = giant_wanted(r->longest[v], r->g_giant[v]);
+    for (uint32_t v = 0; v < r->views; ++v) r->g_giant[v] = view_giant(r, v);
     r->g_whole = r->whole;
     r->g_heads.resize(r->views);
     for (uint32_t v = 0; v < r->views; ++v) r->g_heads[v] = view_heads(r, v);
@@ -551,7 +557,7 @@ int build_graph(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, int
 // Whether some view's choice of the segmented sort differs from the graph's.
 bool giant_changed(const sf_round_t* r) {
     for (uint32_t v = 0; v < r->views; ++v)
-        if (giant_wanted(r->longest[v], r->g_giant[v]) != (r->g_giant[v] != 0)) return true;
+        if (view_giant(r, v) != (r->g_giant[v] != 0)) return true;
     return false;
 }
 
@@ -595,7 +601,7 @@ int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const
             uint64_t total;
             std::memcpy(&total, w + 4, 8);
             worst = std::max(worst, total);
-            r->longest[v] = w[6];
+            r->longest[v] = r->g_heads[v] ? w[7] : w[6];
             if (w[1] & SF_DEV_ERR_CAPACITY) over = true;
             // The heads' cuts move a little from run to run (their sample does).
             need = std::max<uint64_t>(need, r->g_heads[v] ? w[2] + w[2] / 16 : total);

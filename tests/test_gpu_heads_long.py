@@ -1,0 +1,49 @@
+"""Rounds whose heads or whole lists are long enough for the segmented sort
+(GPU): which call captures it, and the per-view path's words in every call."""
+import numpy as np
+import pytest
+
+import splatfield_b200 as sf
+from splatfield_b200 import synth
+from splatfield_b200._lib import lib
+
+pytestmark = pytest.mark.gpu
+
+SIZE = (512, 512)
+
+
+def patch_scene(n, edge):
+    """Nine splats of ten in a slab of `edge` in front of the camera, faint and
+    of a pixel or two; the others anywhere."""
+    attr, sh = synth.scene_uniform(n, 1, seed=29)
+    a = attr.reshape(11, n).copy()
+    m = 9 * n // 10
+    a[0:2, :m] *= 0.5 * edge
+    a[2, :m] *= 0.2
+    a[7:10] -= 2.0
+    a[10] = -2.9
+    return a, sh
+
+
+def run(a, sh, calls):
+    """Kernel launches of each call, whose words it checks."""
+    n = a.shape[1]
+    splats, cam = sf.Splats(a.reshape(-1), sh), sf.look_at((0.0, 0.0, -3.0), (0.0, 0.0, 0.0))
+    scratch, acc = sf.RenderScratch(n, SIZE), sf.Accumulators(n)
+    splats.render_responsibility(scratch, acc, cam, SIZE)
+    want = acc.bits.read()
+    rnd, launched = sf.Round(n, [SIZE]), []
+    for _ in range(calls):
+        before = lib().sf_kernel_launches()
+        rnd.eig(splats, None, [cam])
+        launched.append(lib().sf_kernel_launches() - before)
+        np.testing.assert_array_equal(rnd.responsibility(0)[0].read(), want)
+    return launched
+
+
+def test_whole_lists_after_heads_take_the_segmented_sort_at_once(ctx):
+    """Heads leave 36 tiles open, 16 of them with lists of 27000 to 41700 entries
+    (oracle): the second call takes whole lists, with the seven launches of
+    their segmented sort."""
+    first, second, third = run(*patch_scene(1_000_000, 0.4), 3)
+    assert first != second == third
