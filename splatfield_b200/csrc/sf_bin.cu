@@ -331,6 +331,17 @@ constexpr uint32_t kHeadMinSplats = 640000, kHeadMinTiles = 1024, kHeadSplats = 
 constexpr uint32_t kHeadMaxTiles = 12288;  // limits and counters of a block: 96 KB
 constexpr unsigned long long kMaxPairs = (1ull << 30) - 1;  // of a frame's whole lists
 
+__device__ __forceinline__ void st_relaxed(uint32_t* p, uint32_t v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+
+// A 32-bit mix (the finalizer of MurmurHash3).
+__device__ __forceinline__ uint32_t mix32(uint32_t x) {
+    x = (x ^ (x >> 16)) * 0x85ebca6bu;
+    x = (x ^ (x >> 13)) * 0xc2b2ae35u;
+    return x ^ (x >> 16);
+}
+
 __global__ __launch_bounds__(256) void head_sample_kernel(const uint2* __restrict__ bbox,
                                                           const uint32_t* __restrict__ depth_keys, uint32_t n,
                                                           uint32_t tiles_x, HeadState h) {
@@ -344,8 +355,12 @@ __global__ __launch_bounds__(256) void head_sample_kernel(const uint2* __restric
         key = depth_keys[i];
     }
     spread_pairs<1>(bb, key, tiles_x, [&](uint32_t, uint32_t t, uint32_t kk) {
-        const uint32_t slot = atomicAdd(h.sampled + 8 * (size_t)t, 1u);
-        if (slot < kHeadSamples) h.keys[(size_t)t * kHeadSamples + slot] = kk;
+        // Past kHeadSamples the new key takes the place of a kept one, or not,
+        // at random (reservoir sampling): the first to come are the lowest
+        // splat ids, which in a scene stored in order are all near or all far.
+        uint32_t slot = atomicAdd(h.sampled + 8 * (size_t)t, 1u);
+        if (slot >= kHeadSamples) slot = __umulhi(mix32(slot + t * 0x9e3779b9u), slot + 1u);
+        if (slot < kHeadSamples) st_relaxed(h.keys + (size_t)t * kHeadSamples + slot, kk);
     });
 }
 
