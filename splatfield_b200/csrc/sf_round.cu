@@ -136,13 +136,18 @@ struct sf_round_t {
     std::vector<uint32_t> longest;
     std::vector<uint8_t> g_giant;
     // Views whose heads left more than one in 128 of their tiles unsaturated
-    // (faint splats, a thin scene): they take whole lists until the splats
-    // change (8 views of 1M splats of opacity 0.05: 1.94 ms with whole lists,
-    // 2.22 ms with heads whose tails some tiles want). g_whole: as
-    // captured.
+    // (faint splats, a thin scene): they take whole lists (8 views of 1M splats
+    // of opacity 0.05: 1.94 ms with whole lists, 2.22 ms with heads whose tails
+    // some tiles want). A view is a slot whose camera may be another in the
+    // next round, and a change costs a capture (5 ms), so that is decided where
+    // it says something of later rounds: of half the views with heads, or of
+    // cameras that stay. It lapses after whole_left rounds (kWholeRounds, twice
+    // as many each time), or with the splats. g_whole: as captured.
     std::vector<uint8_t> whole, g_whole;
+    uint32_t whole_left = 0, whole_rounds = 0;
+    uint64_t whole_splats = 0;       // id
+    std::vector<sf_view> last_views;  // of the last round
     std::vector<uint8_t> g_heads;  // views captured with depth-limited lists
-    uint64_t whole_splats = 0;  // id
     uint32_t chunks = 1;
     std::vector<uint64_t> g_masks;  // ids (0: no mask)
 };
@@ -561,12 +566,36 @@ bool giant_changed(const sf_round_t* r) {
     return false;
 }
 
+// After a round: which views take whole lists from the next one on.
+constexpr uint32_t kWholeRounds = 64, kWholeRoundsMost = 1024;
+void settle_heads(sf_round_t* r) {
+    if (r->whole_left && --r->whole_left == 0) r->whole.assign(r->views, 0);
+    std::vector<uint32_t> open;
+    uint32_t heads = 0;
+    for (uint32_t v = 0; v < r->views; ++v) {
+        if (!r->g_heads[v]) continue;
+        ++heads;
+        if (r->words_host[16 * v + 3] > ((r->w[v] + 15) / 16) * ((r->h[v] + 15) / 16) / 128) open.push_back(v);
+    }
+    const bool same = r->last_views.size() == r->views &&
+                      std::memcmp(r->last_views.data(), r->views_host, sizeof(sf_view) * r->views) == 0;
+    if (!same) r->last_views.assign(r->views_host, r->views_host + r->views);
+    if (open.empty() || (!same && 2 * open.size() < heads)) return;
+    for (uint32_t v : open) r->whole[v] = 1;
+    if (r->whole_left == 0) {
+        r->whole_left = r->whole_rounds;
+        r->whole_rounds = std::min(2 * r->whole_rounds, kWholeRoundsMost);
+    }
+}
+
 // Launch the round (rebuilding buffers/graph when needed), wait, check.
 int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const sf_camera* cams, int mode,
               cudaStream_t user) {
     for (uint32_t v = 0; v < r->views; ++v) view_for_camera(cams[v], r->w[v], r->h[v], &r->views_host[v]);
     if (r->whole_splats != sp->id) {
         r->whole.assign(r->views, 0);
+        r->whole_left = 0;
+        r->whole_rounds = kWholeRounds;
         r->whole_splats = sp->id;
     }
     // Heads may outgrow the capacity, then the tails that they leave.
@@ -610,8 +639,7 @@ int run_round(sf_round_t* r, const sf_splats_t* sp, const sf_beta_t* beta, const
         // depend on the form of its lists.
         if (worst > (1ull << 30) - 1) return rfail(SF_ERR_CAPACITY, "intersection count exceeds 2^30-1");
         if (!over) {
-            for (uint32_t v = 0; v < r->views; ++v)
-                if (r->words_host[16 * v + 3] > ((r->w[v] + 15) / 16) * ((r->h[v] + 15) / 16) / 128) r->whole[v] = 1;
+            settle_heads(r);
             return SF_OK;
         }
         r->want_cap = std::max(r->want_cap, std::min<uint64_t>(next_pow2(need), 1ull << 30));

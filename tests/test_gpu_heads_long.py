@@ -61,3 +61,49 @@ def test_heads_of_splats_stored_in_depth_order(ctx, order):
     a[0:2] *= 0.6
     a[2] = np.sort(a[2])[::order]
     assert len(set(run(a, sh, 6))) == 1
+
+
+FAINT = sf.look_at((20.0, 0.0, -3.0), (20.0, 0.0, 0.0))
+
+
+def two_scenes():
+    """650k splats whose heads suffice and, beside them in view of FAINT alone,
+    300k that leave some 36 tiles open."""
+    attr, sh = synth.scene_clustered(650_000, 1, seed=17)
+    faint, sh2 = patch_scene(300_000, 0.4)
+    faint[0] += 20.0
+    a = np.concatenate([attr.reshape(11, -1), faint], axis=1)
+    return sf.Splats(a.reshape(-1), np.concatenate([sh.reshape(3, -1), sh2.reshape(3, -1)], axis=1).reshape(-1))
+
+
+def rounds(splats, cams_of, calls):
+    n, launched = splats.n, []
+    rnd = sf.Round(n, [SIZE] * 3)
+    for k in range(calls):
+        before = lib().sf_kernel_launches()
+        rnd.eig(splats, None, cams_of(k))
+        launched.append(lib().sf_kernel_launches() - before)
+        v = k % 3
+        if k > 6:
+            continue
+        scratch, acc = sf.RenderScratch(n, SIZE), sf.Accumulators(n)
+        splats.render_responsibility(scratch, acc, cams_of(k)[v], SIZE)
+        np.testing.assert_array_equal(rnd.responsibility(v)[0].read(), acc.bits.read())
+    return launched
+
+
+def test_a_passing_faint_view_leaves_its_slot_on_heads(ctx):
+    """The faint camera is in another slot each round."""
+    near = [sf.look_at((0.2 * j, 0.1, -3.5), (0.0, 0.0, 0.0)) for j in range(3)]
+    launched = rounds(two_scenes(), lambda k: [FAINT if j == k % 3 else near[j] for j in range(3)], 6)
+    assert len(set(launched)) == 1
+
+
+def test_a_lasting_faint_view_takes_whole_lists_for_some_rounds(ctx):
+    """From the second round of the same cameras on, for 64 rounds, then heads
+    are tried once and 128 rounds follow."""
+    near = [sf.look_at((0.2 * j, 0.1, -3.5), (0.0, 0.0, 0.0)) for j in range(3)]
+    launched = rounds(two_scenes(), lambda k: [near[0], FAINT, near[2]], 2 + 64 + 1 + 128 + 1)
+    heads, whole = launched[0], launched[2]
+    assert heads > whole
+    assert launched == [heads] * 2 + [whole] * 64 + [heads] + [whole] * 128 + [heads]
