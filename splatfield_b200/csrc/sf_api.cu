@@ -225,6 +225,16 @@ cudaError_t ensure_lut(sf_ctx ctx) {
     return cudaMemcpy(ctx->lut, t.data(), t.size() * 4, cudaMemcpyHostToDevice);
 }
 
+// No prepared frame and no forward state: before a frame starts to overwrite
+// the last one's buffers (it may fail on the way).
+void forget_frame(sf_scratch s) {
+    s->order = nullptr;
+    s->tids = s->gids = nullptr;
+    s->lazy = false;
+    s->prepared = false;
+    s->has_forward = false;
+}
+
 // The captured frame holds the buffers' addresses: it goes before they do.
 void frame_graph_drop(sf_scratch s) {
     if (s->fg.exec) cudaGraphExecDestroy(s->fg.exec);
@@ -241,9 +251,7 @@ void scratch_free_frame(sf_scratch s) {
     dfree(s->giant.taken); dfree(s->giant.segs);
     s->giant.lists = s->giant.seg_cap = 0;
     dfree(s->rgba); dfree(s->final_t); dfree(s->n_contrib); dfree(s->d2d);
-    s->order = nullptr;
-    s->prepared = false;
-    s->has_forward = false;
+    forget_frame(s);
 }
 
 void scratch_free_isects(sf_scratch s) {
@@ -269,6 +277,8 @@ cudaError_t ensure_sort_tmp(sf_scratch s, size_t bytes) {
 cudaError_t grow_isects(sf_scratch s, uint64_t want) {
     if (want <= s->cap && s->tid_e) return cudaSuccess;
     frame_graph_drop(s);
+    s->tids = s->gids = nullptr;
+    s->prepared = s->has_forward = false;
     const uint64_t cap = std::min<uint64_t>(std::max<uint64_t>(next_pow2(want), 1024), kMaxIsects + 1);
     dfree(s->tid_e); dfree(s->gid_e); dfree(s->tid_a);
     s->gid_a = nullptr;
@@ -421,7 +431,7 @@ int prepare(sf_splats sp, sf_scratch s, const sf_camera* cam, uint32_t w, uint32
     if (w == 0 || h == 0 || w > 65535 * 16 || h > 65535 * 16) return fail(SF_ERR_SHAPE, "bad image size");
     SF_CK(use_device(s->ctx->device));
     if (s->total != sp->n || s->w != w || s->h != h) SF_CK(scratch_build(s, sp->n, w, h));
-    s->has_forward = false;
+    forget_frame(s);
     sf_view view;
     view_for_camera(*cam, w, h, &view);
     const uint32_t n = sp->n;
@@ -431,9 +441,6 @@ int prepare(sf_splats sp, sf_scratch s, const sf_camera* cam, uint32_t w, uint32
     ProjOut po{s->depth_keys, s->tile_counts, s->bbox, s->geo0, s->geo1, s->color, words, s->ext};
     SF_CK(launch_project(view, sp->attr, sp->geom, sp->sh, n, sp->K, po, st));
     const uint32_t tiles = s->tiles_x * s->tiles_y;
-    s->order = nullptr;
-    s->tids = s->gids = nullptr;
-    s->lazy = false;
     if (s->tuning.isect_build == SF_ISECTS_BINNED && s->bin_hist) {
         const int rc = prepare_binned(s, n, tiles, st, out != nullptr,
                                       (lazy && out == nullptr) ? s->tuning.raster_order : SF_ORDER_SORTED);
@@ -713,6 +720,7 @@ void frame_graph_settle(sf_scratch s, const uint32_t* hw, uint64_t total) {
 int frame_graph_render(sf_splats sp, sf_scratch s, const sf_camera* cam, uint32_t w, uint32_t h,
                        cudaStream_t st, uint32_t* host_out) {
     auto& g = s->fg;
+    forget_frame(s);
     for (int attempt = 0; attempt < 4; ++attempt) {
         const int rc = frame_graph_ready(sp, s);
         if (rc != SF_OK) return rc;
@@ -835,6 +843,7 @@ int frames_graph_render(sf_splats sp, sf_scratch s, const sf_camera* cams, uint3
     auto& g = s->fg;
     const size_t img = (size_t)w * h;
     bool two = count >= 2 && s->tuning.frame_pipes != 1;
+    forget_frame(s);
     int rc = frame_graph_ready(sp, s);
     if (rc != SF_OK) return rc;
     if (two && (rc = twin_ready(sp, s, w, h)) != SF_OK) {
@@ -1222,6 +1231,7 @@ int sf_finalize_rgb(sf_splats s, sf_scratch scratch, const sf_isects* isects, ui
         if (!s || !scratch || !isects) return fail(SF_ERR_ARG, "null argument");
         if (!scratch->prepared || scratch->w != w || scratch->h != h)
             return fail(SF_ERR_SHAPE, "finalize without a matching prepare");
+        if (scratch->lazy) return fail(SF_ERR_ARG, "the scratch's last frame left no sorted lists");
         return finalize_rgb(scratch, isects, want_float != 0, S(stream));
     })
 }
@@ -1688,6 +1698,7 @@ int sf_accumulate_prepared(sf_splats s, sf_scratch scratch, const sf_isects* ise
         if (!s || !scratch || !isects || !acc) return fail(SF_ERR_ARG, "null argument");
         if (!scratch->prepared || scratch->w != w || scratch->h != h)
             return fail(SF_ERR_SHAPE, "accumulate without a matching prepare");
+        if (scratch->lazy) return fail(SF_ERR_ARG, "the scratch's last frame left no sorted lists");
         SF_CK(use_device(scratch->ctx->device));
         return accumulate(scratch, isects, w, h, acc, mask, S(stream));
     })
