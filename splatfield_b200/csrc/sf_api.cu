@@ -290,12 +290,14 @@ cudaError_t grow_isects(sf_scratch s, uint64_t want) {
     // (depth key, splat id) pairs across both.
     if ((e = dalloc(&s->tid_a, 2 * cap)) != cudaSuccess) return e;
     s->gid_a = s->tid_a + cap;
+    if ((e = ensure_sort_tmp(s, std::max(radix_temp_bytes((uint32_t)std::min<uint64_t>(cap, kMaxIsects), 4),
+                                         radix_temp_bytes(s->total, 4)))) != cudaSuccess)
+        return e;
     s->cap = cap;
-    return ensure_sort_tmp(s, std::max(radix_temp_bytes((uint32_t)std::min<uint64_t>(cap, kMaxIsects), 4),
-                                       radix_temp_bytes(s->total, 4)));
+    return cudaSuccess;
 }
 
-cudaError_t scratch_build(sf_scratch s, uint32_t total, uint32_t w, uint32_t h) {
+cudaError_t scratch_alloc(sf_scratch s, uint32_t total, uint32_t w, uint32_t h) {
     scratch_free_frame(s);
     s->total = total;
     s->w = w;
@@ -353,6 +355,18 @@ cudaError_t scratch_build(sf_scratch s, uint32_t total, uint32_t w, uint32_t h) 
     // frame rule min(tiles*total, 2^22) (render.rs:146-147, 177-183).
     const uint64_t first = std::min<uint64_t>((uint64_t)s->tiles_x * s->tiles_y * total, kInitialIsects);
     return grow_isects(s, std::max<uint64_t>(std::max<uint64_t>(first, s->last_isects_raw), s->cap));
+}
+
+// The scratch at another size; one that does not fit leaves it at none (the
+// next call builds it anew).
+cudaError_t scratch_build(sf_scratch s, uint32_t total, uint32_t w, uint32_t h) {
+    const cudaError_t e = scratch_alloc(s, total, w, h);
+    if (e != cudaSuccess) {
+        scratch_free_frame(s);
+        s->w = s->h = 0;
+        cudaGetLastError();
+    }
+    return e;
 }
 
 int finish_prepare(sf_scratch s, sf_isects* out);

@@ -245,7 +245,13 @@ cudaError_t lanes_build(sf_round_t* r, uint32_t lanes, uint64_t cap) {
     r->lanes.assign(lanes, RoundLane());
     for (auto& L : r->lanes) {
         cudaError_t e = lane_alloc(r, L, cap);
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess) {
+            // None rather than some: the next round builds them anew.
+            for (auto& M : r->lanes) lane_free(M);
+            r->lanes.clear();
+            cudaGetLastError();
+            return e;
+        }
     }
     return cudaSuccess;
 }
