@@ -340,8 +340,7 @@ cudaError_t scratch_alloc(sf_scratch s, uint32_t total, uint32_t w, uint32_t h) 
     // Row padding (row_stride past w) is never rendered: clear it once so
     // read-backs of whole rows are deterministic.
     if ((e = cudaMemset(s->bitmap, 0, (size_t)h * s->row_stride * 4)) != cudaSuccess) return e;
-    const uint32_t scan_n = (uint32_t)std::max<size_t>(total, tiles + 1);
-    if ((e = cudaMalloc(&s->scan_tmp, scan_temp_bytes(scan_n))) != cudaSuccess) return e;
+    if ((e = cudaMalloc(&s->scan_tmp, scan_temp_bytes(total))) != cudaSuccess) return e;
     if (!s->words) {
         // One block, cleared together at the start of a frame graph.
         if ((e = dalloc(&s->words, kStatusWords)) != cudaSuccess) return e;
@@ -396,7 +395,6 @@ int prepare_binned(sf_scratch s, uint32_t n, uint32_t tiles, cudaStream_t st, bo
     SF_CK(place());
     SF_CK(cudaStreamSynchronize(side));
     const uint32_t* hw = s->host_words;
-    if (hw[1] & SF_DEV_ERR_TIMEOUT) return fail(SF_ERR_TIMEOUT, "device look-back wait timed out");
     uint64_t total = 0;
     std::memcpy(&total, hw + 4, 8);
     s->num_visible = hw[0];
@@ -747,7 +745,6 @@ int frame_graph_render(sf_splats sp, sf_scratch s, const sf_camera* cam, uint32_
                                     h, cudaMemcpyDeviceToHost, st));
         SF_CK(cudaStreamSynchronize(st));
         const uint32_t* hw = s->host_words;
-        if (hw[1] & SF_DEV_ERR_TIMEOUT) return fail(SF_ERR_TIMEOUT, "device look-back wait timed out");
         uint64_t total = 0;
         std::memcpy(&total, hw + 4, 8);
         s->num_visible = hw[0];
@@ -926,7 +923,6 @@ int frames_graph_render(sf_splats sp, sf_scratch s, const sf_camera* cams, uint3
     bool over = false;
     for (uint32_t i = 0; i < count; ++i) {
         const uint32_t* hw = g.frame_words + 16 * (size_t)i;
-        if (hw[1] & SF_DEV_ERR_TIMEOUT) return fail(SF_ERR_TIMEOUT, "device look-back wait timed out");
         uint64_t total = 0;
         std::memcpy(&total, hw + 4, 8);
         if (total > kMaxIsects) return fail(SF_ERR_CAPACITY, "intersection count exceeds 2^30-1");

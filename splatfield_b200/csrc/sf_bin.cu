@@ -51,62 +51,62 @@ template <uint32_t U, typename F>
 __device__ __forceinline__ void spread_pairs(const uint2 bb, const uint32_t pay, uint32_t tiles_x, F&& f,
                                              unsigned long long* pairs = nullptr) {
     const uint32_t lane = threadIdx.x & 31u;
-            uint32_t min_x = bb.x & 0xffffu, min_y = bb.x >> 16, width = 1, cnt = 0;
-            const uint32_t max_x = bb.y & 0xffffu, max_y = bb.y >> 16;
-            if (max_x > min_x && max_y > min_y) {
-                width = max_x - min_x;
-                cnt = width * (max_y - min_y);
+    uint32_t min_x = bb.x & 0xffffu, min_y = bb.x >> 16, width = 1, cnt = 0;
+    const uint32_t max_x = bb.y & 0xffffu, max_y = bb.y >> 16;
+    if (max_x > min_x && max_y > min_y) {
+        width = max_x - min_x;
+        cnt = width * (max_y - min_y);
+    }
+    if (pairs) *pairs += cnt;
+    // 1 / width, shuffled to the pair lanes with the box.
+    const float rw = __fdividef(1.0f, (float)width);
+    uint32_t incl = cnt;
+#pragma unroll
+    for (uint32_t d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += v;
+    }
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    for (uint32_t p0 = 0; p0 < total; p0 += 32u * U) {
+        uint32_t o[U];
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) o[u] = 0;
+#pragma unroll
+        for (uint32_t step = 16; step > 0; step >>= 1) {
+#pragma unroll
+            for (uint32_t u = 0; u < U; ++u) {
+                const uint32_t v = __shfl_sync(0xffffffffu, incl, o[u] + step - 1);
+                if (v <= p0 + 32u * u + lane) o[u] += step;
             }
-            if (pairs) *pairs += cnt;
-            // 1 / width, shuffled to the pair lanes with the box.
-            const float rw = __fdividef(1.0f, (float)width);
-            uint32_t incl = cnt;
-    #pragma unroll
-            for (uint32_t d = 1; d < 32; d <<= 1) {
-                const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-                if (lane >= d) incl += v;
-            }
-            const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-            for (uint32_t p0 = 0; p0 < total; p0 += 32u * U) {
-                uint32_t o[U];
-    #pragma unroll
-                for (uint32_t u = 0; u < U; ++u) o[u] = 0;
-    #pragma unroll
-                for (uint32_t step = 16; step > 0; step >>= 1) {
-    #pragma unroll
-                    for (uint32_t u = 0; u < U; ++u) {
-                        const uint32_t v = __shfl_sync(0xffffffffu, incl, o[u] + step - 1);
-                        if (v <= p0 + 32u * u + lane) o[u] += step;
-                    }
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < U; ++u) {
+            const uint32_t p = p0 + 32u * u + lane;
+            const uint32_t oend = __shfl_sync(0xffffffffu, incl, o[u]);
+            const uint32_t ocnt = __shfl_sync(0xffffffffu, cnt, o[u]);
+            const uint32_t ow = __shfl_sync(0xffffffffu, width, o[u]);
+            const float orw = __shfl_sync(0xffffffffu, rw, o[u]);
+            const uint32_t ox = __shfl_sync(0xffffffffu, min_x, o[u]);
+            const uint32_t oy = __shfl_sync(0xffffffffu, min_y, o[u]);
+            const uint32_t opay = __shfl_sync(0xffffffffu, pay, o[u]);
+            if (p < total) {
+                // Row and column of pair k in the owner's box: a float
+                // quotient (k < 2^16, so it is off by at most one) and an
+                // exact integer correction.
+                const uint32_t k = p - (oend - ocnt);
+                uint32_t row = (uint32_t)((float)k * orw);
+                int32_t col = (int32_t)(k - row * ow);
+                if (col < 0) {
+                    --row;
+                    col += (int32_t)ow;
+                } else if (col >= (int32_t)ow) {
+                    ++row;
+                    col -= (int32_t)ow;
                 }
-    #pragma unroll
-                for (uint32_t u = 0; u < U; ++u) {
-                    const uint32_t p = p0 + 32u * u + lane;
-                    const uint32_t oend = __shfl_sync(0xffffffffu, incl, o[u]);
-                    const uint32_t ocnt = __shfl_sync(0xffffffffu, cnt, o[u]);
-                    const uint32_t ow = __shfl_sync(0xffffffffu, width, o[u]);
-                    const float orw = __shfl_sync(0xffffffffu, rw, o[u]);
-                    const uint32_t ox = __shfl_sync(0xffffffffu, min_x, o[u]);
-                    const uint32_t oy = __shfl_sync(0xffffffffu, min_y, o[u]);
-                    const uint32_t opay = __shfl_sync(0xffffffffu, pay, o[u]);
-                    if (p < total) {
-                        // Row and column of pair k in the owner's box: a float
-                        // quotient (k < 2^16, so it is off by at most one) and an
-                        // exact integer correction.
-                        const uint32_t k = p - (oend - ocnt);
-                        uint32_t row = (uint32_t)((float)k * orw);
-                        int32_t col = (int32_t)(k - row * ow);
-                        if (col < 0) {
-                            --row;
-                            col += (int32_t)ow;
-                        } else if (col >= (int32_t)ow) {
-                            ++row;
-                            col -= (int32_t)ow;
-                        }
-                        f(o[u], (ox + (uint32_t)col) + (oy + row) * tiles_x, opay);
-                    }
-                }
+                f(o[u], (ox + (uint32_t)col) + (oy + row) * tiles_x, opay);
             }
+        }
+    }
 }
 
 // Calls f(splat, tile, payload) for every tile of every splat in [begin,
@@ -322,7 +322,11 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t x, uint32_t* s32, uint32
 // views included). Where the lists are short or the tiles few, the six more
 // kernels of a view are not repaid: 12 views of 512 squared of 530k splats
 // 1.19 -> 1.21 ms, of 256 squared of 300k 0.93 -> 1.20 ms, of 200 squared of
-// 1M 2.27 -> 3.05 ms; hence heads_wanted.
+// 1M 2.27 -> 3.05 ms; hence heads_wanted. Between 400 and 1024 tiles it is the
+// lists that decide, and the line at 1024 leaves gains of long ones aside: 12
+// views of 320, 384 and 448 squared of 650k splats 1.32 -> 1.39, 1.13 -> 1.21
+// and 1.29 -> 1.46 ms, of 1M 1.74 -> 1.58, 1.72 -> 1.48 and 1.75 -> 1.75, of 3M
+// 4.41 -> 4.05, 4.34 -> 3.34 and 4.42 -> 3.26.
 constexpr uint32_t kHeadStride = 32;     // splats per sampled splat
 static_assert(kHeadStride == 32, "the sample's place is five bits");
 constexpr uint32_t kHeadTarget = 2048;   // pairs aimed at

@@ -224,7 +224,7 @@ cudaError_t lane_alloc(sf_round_t* r, RoundLane& L, uint64_t cap) {
         H.t = reinterpret_cast<float*>(H.list + head_tiles);
     }
 #undef RA
-    if ((e = cudaMalloc(&L.scan_tmp, scan_temp_bytes(std::max(n, r->max_tiles + 1)))) != cudaSuccess) return e;
+    if ((e = cudaMalloc(&L.scan_tmp, scan_temp_bytes(n))) != cudaSuccess) return e;
     const size_t st = std::max(radix_temp_bytes(n, 4), radix_temp_bytes((uint32_t)cap, 4));
     if ((e = cudaMalloc(&L.sort_tmp, st)) != cudaSuccess) return e;
     if ((e = cudaStreamCreateWithFlags(&L.stream, cudaStreamNonBlocking)) != cudaSuccess) return e;
