@@ -299,7 +299,9 @@ int sf_render_feature_adjoint(sf_splats s, sf_scratch scratch, const sf_camera* 
 int sf_prepare_isects(sf_splats s, sf_scratch scratch, const sf_camera* cam, uint32_t w, uint32_t h,
                       sf_stream stream, sf_isects* out);
 /* Splats::finalize(Finalize::Rgb) (src/render.rs:387-460) over prepared
- * intersections; optionally also the float plane. */
+ * intersections; optionally also the float plane. An error where the scratch
+ * has no lists: its last call failed, sf_scratch_reserve has grown it since, or
+ * its last frame ordered them in the rasterizer. */
 int sf_finalize_rgb(sf_splats s, sf_scratch scratch, const sf_isects* isects, uint32_t w,
                     uint32_t h, int want_float, sf_stream stream);
 
@@ -359,7 +361,8 @@ int sf_render_responsibility(sf_splats s, sf_scratch scratch, sf_accum acc, cons
                              uint32_t w, uint32_t h, sf_stream stream);
 /* Splats::accumulate_prepared (src/seg/mod.rs:170-210): over intersections
  * already prepared for this camera and size; mask NULL = total
- * responsibility, else the fg/bg evidence split. */
+ * responsibility, else the fg/bg evidence split. Refused where
+ * sf_finalize_rgb is. */
 int sf_accumulate_prepared(sf_splats s, sf_scratch scratch, const sf_isects* isects, uint32_t w,
                            uint32_t h, sf_accum acc, sf_mask mask, sf_stream stream);
 /* fractional_bits (src/seg/mod.rs:31-34) and the scale 2^bits. */

@@ -876,7 +876,7 @@ int round_of_kind(sf_round r, sf_splats s, sf_beta beta, const sf_camera* cams, 
 }
 
 // Coordinate search over the round's kernel forms: each dimension in turn
-// (lanes, intersection build, list order, raster culling, CTAs per tile),
+// (lanes, intersection build, list order, CTAs per tile, digit width),
 // each value timed as the best of three rounds after one warm-up round
 // (which also captures the graph), the best kept; two sweeps.
 int autotune(sf_round r, sf_splats s, sf_beta beta, const sf_camera* cams, const sf_mask* masks, int kind,
